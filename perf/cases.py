@@ -327,3 +327,67 @@ def run(state):
         model.forward(token, position, fetch=every)
     token, position = feed[-1]
     return model.forward(token, position)
+
+
+# ---- the same in 64 bits -----------------------------------------------------------------------------------
+
+def _unpack(raw, bits):
+    """[..., bytes] of a most-significant-bit-first stream as [..., codes] of `bits` bits each."""
+    planes = torch.stack([(raw >> (7 - i)) & 1 for i in range(8)], dim=-1).flatten(-2)
+    codes = planes.unflatten(-1, (-1, bits)).double()
+    return codes @ torch.tensor([float(1 << (bits - 1 - i)) for i in range(bits)], dtype=torch.float64, device=raw.device)
+
+
+def _dense(t):
+    """The weights of a tensor as fp64 [M, padded K]."""
+    def part(name):
+        a = np.ascontiguousarray(t.blocks[name])
+        return torch.from_numpy(a.view(np.uint8) if a.dtype == np.int8 else a.copy()).to(DEVICE)
+
+    s = part("scale").double()[:, None]
+    if t.kind == TERNARY:
+        w = (1 - _unpack(part("zero_plane"), 1)) * (1 - 2 * _unpack(part("sign_plane"), 1)) * s
+    elif t.kind == BINARY:
+        w = (2 * _unpack(part("data"), 1) - 1) * s
+    elif t.kind == INT2:
+        b = _unpack(part("data"), 1).unflatten(-1, (-1, 2))
+        w = (2 * b[..., 0] - 1) * s + (2 * b[..., 1] - 1) * part("scale2").double()[:, None]
+    elif t.kind == INT8:
+        w = part("data").view(torch.int8).double() * s
+    else:
+        w = (_unpack(part("data"), t.kind) - float(1 << (t.kind - 1))) * s
+    return w.view(t.M, -1)
+
+
+def _linear_exact(t, x, batch, bias=None):
+    xs = torch.zeros(batch, blocks_per_row(t.K) * 256, dtype=torch.float64, device=DEVICE)
+    xs[:, :t.K] = torch.from_numpy(x).to(DEVICE).double().view(batch, t.K)
+    if t.kind in (TERNARY, BINARY, INT2):  # these kinds meet inputs rotated by a 256-point Hadamard transform
+        h = torch.ones(1, 1, dtype=torch.float64, device=DEVICE)
+        for _ in range(8):
+            h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+        xs = (xs.view(-1, 256) @ h / 16).view(batch, -1)
+    y = xs @ _dense(t).T
+    return y if bias is None else y + torch.from_numpy(bias).to(DEVICE).double()
+
+
+def exact(case, seed):
+    """What run() returns in 64 bits, for the projections; the quantizers' and decode steps' own arithmetic has
+    oracles in the tests."""
+    r = _Random(seed)
+    if case["op"] == "linear":
+        t = _tensor(r, KINDS[case["kind"]], case["M"], case["K"])
+        x = r.activations(case["batch"] * case["K"])
+        return _linear_exact(t, x, case["batch"], r.normal(case["M"]).cpu().numpy() if case["bias"] else None)
+    if case["op"] == "host":
+        t = _tensor(r, KINDS[case["kind"]], case["M"], case["K"])
+        x = r.activations(case["batch"] * case["K"])
+        return _linear_exact(t, x, case["batch"], r.normal(case["M"]).cpu().numpy() if case["bias"] else None).flatten().cpu().numpy()
+    if case["op"] == "group":
+        out = []
+        for _ in range(case["layers"]):
+            for _, M, K in _projections(synth.MODEL_SHAPES[case["shape"]]):
+                t = _tensor(r, KINDS[case["kind"]], M, K)
+                out.append(_linear_exact(t, r.activations(K), 1).flatten())
+        return out
+    return None

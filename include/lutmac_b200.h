@@ -225,6 +225,9 @@ int lmb_debug_plan_weight(const lmb_weight *w, int sm_count, int out5[5]);
  * cr * n_ks in {2, 4, 8}, cr = 0: no cluster); launches that cannot, plan as usual.  R = 0: off.
  * Process-wide; graphs captured earlier keep their plans. */
 int lmb_debug_force_plan(int R, int n_ks, int cr);
+/* Tests: from now on the batched projections' operand barriers expect `extra_arrivals` arrivals too many
+ * and their waits give up after `spin_limit` polls (0: the default); 0, 0: off. */
+int lmb_debug_batched_waits(lmb_ctx *ctx, int extra_arrivals, unsigned spin_limit);
 /* Range-checking build (liblutmac_b200_dbg.so, compiled with -DLMB_DEBUG_BOUNDS; the reference has no
  * sanitizer set-up to mirror): the GEMV kernels check every weight-tile load, output store and
  * split-K scratch store against the extent of its buffer, the attention kernel its cache slices; an

@@ -47,6 +47,40 @@ int ensure_scratch(lmb_ctx *ctx, size_t floats, size_t counters) {
   return LMB_OK;
 }
 
+// A launch that left early may have left arrival counters behind: they start from zero again.
+int clear_fault(lmb_ctx *ctx) {
+  LMB_CUDA(cudaMemsetAsync(ctx->d_fault, 0, sizeof(unsigned), ctx->stream));
+  LMB_CUDA(cudaMemsetAsync(ctx->counters, 0, ctx->n_counters * sizeof(unsigned), ctx->stream));
+  LMB_CUDA(cudaStreamSynchronize(ctx->stream));
+  return LMB_OK;
+}
+
+// After the stream has been waited for: LMB_ERR_TIMEOUT if a batched launch gave up a bounded wait.
+int check_fault(lmb_ctx *ctx, const char *who) {
+  if (!ctx->fault_unread || !ctx->d_fault) return LMB_OK;
+  unsigned v = 0;
+  LMB_CUDA(cudaMemcpyAsync(&v, ctx->d_fault, sizeof v, cudaMemcpyDeviceToHost, ctx->stream));
+  LMB_CUDA(cudaStreamSynchronize(ctx->stream));
+  ctx->fault_unread = false;
+  if (!v) return LMB_OK;
+  int st = clear_fault(ctx);
+  if (st != LMB_OK) return st;
+  set_last_error(std::string(who) + ": a bounded wait for asynchronous copies expired in a kernel");
+  return LMB_ERR_TIMEOUT;
+}
+
+// Prepared activations of batched launches, `blocks` records.  The caller has waited for the stream and is not capturing.
+int ensure_xprep(lmb_ctx *ctx, size_t blocks) {
+  if (blocks <= ctx->xprep_blocks) return LMB_OK;
+  if (ctx->xprep) LMB_CUDA(cudaFree(ctx->xprep));
+  ctx->xprep = nullptr;
+  ctx->xprep_blocks = 0;
+  LMB_CUDA(cudaMalloc(&ctx->xprep, blocks * PREP_RECORD_WORDS * sizeof(uint32_t)));
+  ctx->xprep_blocks = blocks;
+  ctx->scratch_gen++;
+  return LMB_OK;
+}
+
 int ensure_stage(lmb_ctx *ctx, size_t bytes) {
   if (bytes > ctx->h_stage_bytes) {
     if (ctx->h_stage) LMB_CUDA(cudaFreeHost(ctx->h_stage));
@@ -343,7 +377,7 @@ int lmb_ctx_set_option(lmb_ctx *ctx, int option, int value) {
 int lmb_ctx_sync(lmb_ctx *ctx) {
   LMB_REQUIRE(ctx, "lmb_ctx_sync: null context");
   LMB_CUDA(cudaStreamSynchronize(ctx->stream));
-  return LMB_OK;
+  return check_fault(ctx, "lmb_ctx_sync");
 }
 
 int lmb_ctx_launch_count(lmb_ctx *ctx, uint64_t *out) {
@@ -379,7 +413,7 @@ int lmb_memcpy_d2h(lmb_ctx *ctx, void *h_dst, const void *d_src, size_t bytes) {
   LMB_REQUIRE(ctx && (bytes == 0 || (h_dst && d_src)), "lmb_memcpy_d2h: null argument");
   LMB_CUDA(cudaMemcpyAsync(h_dst, d_src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   LMB_CUDA(cudaStreamSynchronize(ctx->stream));
-  return LMB_OK;
+  return check_fault(ctx, "lmb_memcpy_d2h");
 }
 
 int lmb_memset(lmb_ctx *ctx, void *d_dst, int value, size_t bytes) {
@@ -598,7 +632,7 @@ int lmb_linear_host(lmb_ctx *ctx, const lmb_weight *w, const float *bias, const 
   LMB_REQUIRE(ctx && w && input && output && batch > 0, "lmb_linear_host: null argument");
   const size_t K = w->K, M = w->M;
   const size_t in_f = batch * K, out_f = batch * M, bias_f = bias ? M : 0;
-  int st = ensure_stage(ctx, (in_f + out_f + bias_f) * sizeof(float));
+  int st = ensure_stage(ctx, (in_f + out_f + bias_f + 1) * sizeof(float));
   if (st != LMB_OK) return st;
   float *h = static_cast<float *>(ctx->h_stage), *d = ctx->d_stage;
   std::memcpy(h, input, in_f * sizeof(float));
@@ -609,9 +643,15 @@ int lmb_linear_host(lmb_ctx *ctx, const lmb_weight *w, const float *bias, const 
   if (st != LMB_OK) return st;
   float *h_y = h + in_f + bias_f;
   LMB_CUDA(cudaMemcpyAsync(h_y, d_y, out_f * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+  // the fault flag of a batched launch rides behind the outputs
+  unsigned *h_fault = reinterpret_cast<unsigned *>(h_y + out_f);
+  const bool look = ctx->fault_unread;
+  *h_fault = 0;
+  if (look) LMB_CUDA(cudaMemcpyAsync(h_fault, ctx->d_fault, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
   LMB_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (look && *h_fault == 0) ctx->fault_unread = false;
   std::memcpy(output, h_y, out_f * sizeof(float));
-  return LMB_OK;
+  return check_fault(ctx, "lmb_linear_host");
 }
 
 int lmb_linear_host_multi(lmb_ctx *ctx, size_t n, const lmb_weight *const *ws, const float *const *inputs,

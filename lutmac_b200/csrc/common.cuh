@@ -191,6 +191,9 @@ struct lmb_ctx {
   size_t xprep_blocks = 0;  // capacity in (sequence, block) pairs
   // set by a kernel whose bounded wait (for its own asynchronous copies) ran out; read with the logits
   unsigned *d_fault = nullptr;
+  unsigned batched_spin_limit = 1u << 22;  // polls before a wait of the batched kernel gives up (seconds)
+  int batched_extra_arrivals = 0;          // test hook, lmb_debug_batched_waits
+  bool fault_unread = false;  // a batched launch may have set it since it was last read (lmb_ctx_sync, host entry points)
   // launch timeline (debugging, lmb_debug_launch_timeline): 8 time stamps per launch, null when off
   unsigned long long *d_timeline = nullptr;
   int timeline_cap = 0, timeline_cursor = 0, timeline_used = 0;  // used: most slots any step has taken (graph replays launch nothing)
@@ -265,11 +268,18 @@ enum { XMODE_PLAIN = 0, XMODE_RMSNORM = 1, XMODE_SILU_MUL = 2, XMODE_GELU_MUL = 
 int configure_gemv(lmb_ctx *ctx);
 int launch_tp_sum_prepare(lmb_ctx *ctx, float *d_hidden, const float *d_w, bool rotate, uint32_t *prep, float *sumsq, size_t h);
 int launch_gemv(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, int xmode = XMODE_PLAIN, float eps = 0.0f);
+// Several sequences per launch on tcgen05 (batched.cu); LMB_ERR_LIMIT: not while capturing with these workspaces.
+int configure_batched();
+bool batched_possible(const LinearArgs *args, int njobs);
+int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, int xmode, float eps);
 int launch_fwht256(lmb_ctx *ctx, float *d_x, size_t n);
 int launch_debug_luts(lmb_ctx *ctx, const float *d_x, size_t x_len, bool rotate, float *d_out);
 
 int model_tie_head(lmb_model *m);  // definition of lmb_model_tie_head
 int ensure_scratch(lmb_ctx *ctx, size_t floats, size_t counters);
+int check_fault(lmb_ctx *ctx, const char *who);
+int clear_fault(lmb_ctx *ctx);
+int ensure_xprep(lmb_ctx *ctx, size_t blocks);
 int ensure_stage(lmb_ctx *ctx, size_t bytes);
 
 }  // namespace lmb

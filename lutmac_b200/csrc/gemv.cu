@@ -1016,6 +1016,7 @@ int configure_gemv(lmb_ctx *ctx) {
   if (st == LMB_OK) st = configure_mma<LMB_INT6>();
   if (st == LMB_OK) st = configure_mma<DK_INT8_MMA>();
   if (st == LMB_OK) st = configure_mma<DK_INT3_MMA>();
+  if (st == LMB_OK) st = configure_batched();
   return st;
 }
 
@@ -1055,6 +1056,10 @@ int launch_gemv(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, in
       set_last_error("launch_gemv: jobs of one launch must share block kind and batch size");
       return LMB_ERR_ARG;
     }
+  if (batched_possible(args, njobs)) {
+    const int st = launch_batched(ctx, args, njobs, rotate, xmode, eps);
+    if (st != LMB_ERR_LIMIT) return st;
+  }
   GemvParams p;
   p.njobs = njobs;
   p.rotate = rotate ? 1 : 0;
@@ -1107,12 +1112,8 @@ int launch_gemv(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, in
       LMB_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
       if (cs == cudaStreamCaptureStatusNone) {
         LMB_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (ctx->xprep) LMB_CUDA(cudaFree(ctx->xprep));
-        ctx->xprep = nullptr;
-        ctx->xprep_blocks = 0;
-        LMB_CUDA(cudaMalloc(&ctx->xprep, need * PREP_WORDS * sizeof(uint32_t)));
-        ctx->xprep_blocks = need;
-        ctx->scratch_gen++;
+        st = ensure_xprep(ctx, need);
+        if (st != LMB_OK) return st;
       }
     }
     if (need <= ctx->xprep_blocks) {

@@ -345,8 +345,13 @@ template <> struct Unit<LMB_INT4> : MmaUnitBase<Unit<LMB_INT4>, 4> {
   }
 };
 
-// (definition of the shared MMA prologue)
-__device__ __forceinline__ void mma_prologue(const float (&v)[8], int lane, float *blk, float *bscale, int *aux2) {
+// The fixed-point digits of one 256-block, one warp, lane l holding elements 8l..8l+7.
+struct MmaDigits {
+  uint32_t words[4][2];  // [digit][h]: that digit of the lane's elements 4h..4h+3
+  float bscale;          // 2^(E-30), 0 for an all-zero block
+  int d01, d23;          // sums over the block of digit 0 + 256 digit 1 and digit 2 + 256 digit 3 (all lanes)
+};
+__device__ __forceinline__ void mma_digits(const float (&v)[8], MmaDigits &o) {
   float amax = 0.0f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
@@ -360,34 +365,40 @@ __device__ __forceinline__ void mma_prologue(const float (&v)[8], int lane, floa
   uint32_t w[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) w[j] = (uint32_t(__float2int_rn(v[j] * inv)) + 0x00808080u) ^ 0x00808080u;
-  // 4x4 byte transposes: words[d][h] = digit d of elements 4h..4h+3
-  uint32_t words[4][2];
+  // 4x4 byte transposes
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const uint32_t t0 = __byte_perm(w[4 * h], w[4 * h + 1], 0x5140), t1 = __byte_perm(w[4 * h + 2], w[4 * h + 3], 0x5140);
     const uint32_t t2 = __byte_perm(w[4 * h], w[4 * h + 1], 0x7362), t3 = __byte_perm(w[4 * h + 2], w[4 * h + 3], 0x7362);
-    words[0][h] = __byte_perm(t0, t1, 0x5410);
-    words[1][h] = __byte_perm(t0, t1, 0x7632);
-    words[2][h] = __byte_perm(t2, t3, 0x5410);
-    words[3][h] = __byte_perm(t2, t3, 0x7632);
+    o.words[0][h] = __byte_perm(t0, t1, 0x5410);
+    o.words[1][h] = __byte_perm(t0, t1, 0x7632);
+    o.words[2][h] = __byte_perm(t2, t3, 0x5410);
+    o.words[3][h] = __byte_perm(t2, t3, 0x7632);
   }
+  int ds[4];
+#pragma unroll
+  for (int d = 0; d < 4; ++d) ds[d] = __dp4a(int(o.words[d][0]), 0x01010101, __dp4a(int(o.words[d][1]), 0x01010101, 0));
+  o.d01 = __reduce_add_sync(0xffffffffu, ds[0] + 256 * ds[1]);
+  o.d23 = __reduce_add_sync(0xffffffffu, ds[2] + 256 * ds[3]);
+  o.bscale = (am != 0u) ? __uint_as_float(uint32_t(127 + e - 30) << 23) : 0.0f;
+}
+
+// (definition of the shared MMA prologue)
+__device__ __forceinline__ void mma_prologue(const float (&v)[8], int lane, float *blk, float *bscale, int *aux2) {
+  MmaDigits dg;
+  mma_digits(v, dg);
   // element j of lane l is column 8l+j: k-step s = l/4, position kk = 8(l%4)+j inside it
   const int s = lane >> 2, reg = (lane & 3) >> 1, tidb = 2 * (lane & 1);
   uint32_t *dst = reinterpret_cast<uint32_t *>(blk) + ((s >> 1) * 16 + tidb) * 4 + (s & 1) * 2 + reg;
 #pragma unroll
   for (int d = 0; d < 4; ++d) {
-    dst[d * 16] = words[d][0];
-    dst[d * 16 + 4] = words[d][1];
+    dst[d * 16] = dg.words[d][0];
+    dst[d * 16 + 4] = dg.words[d][1];
   }
-  int ds[4];
-#pragma unroll
-  for (int d = 0; d < 4; ++d) ds[d] = __dp4a(int(words[d][0]), 0x01010101, __dp4a(int(words[d][1]), 0x01010101, 0));
-  const int d01 = __reduce_add_sync(0xffffffffu, ds[0] + 256 * ds[1]);
-  const int d23 = __reduce_add_sync(0xffffffffu, ds[2] + 256 * ds[3]);
   if (lane == 0) {
-    *bscale = (am != 0u) ? __uint_as_float(uint32_t(127 + e - 30) << 23) : 0.0f;
-    aux2[0] = d01;
-    aux2[1] = d23;
+    *bscale = dg.bscale;
+    aux2[0] = dg.d01;
+    aux2[1] = dg.d23;
   }
 }
 

@@ -845,8 +845,9 @@ fetch:
                                cudaMemcpyDeviceToHost, ctx->stream));
     LMB_CUDA(cudaStreamSynchronize(ctx->stream));
     if (hs[0]) {  // a kernel's bounded wait for its own asynchronous copies ran out
-      LMB_CUDA(cudaMemset(ctx->d_fault, 0, sizeof(unsigned)));
-      set_last_error("lmb_model_forward: a bounded wait for asynchronous copies expired in the attention kernel");
+      st = clear_fault(ctx);
+      if (st != LMB_OK) return st;
+      set_last_error("lmb_model_forward: a bounded wait for asynchronous copies expired in the attention kernel or a batched projection");
       return LMB_ERR_TIMEOUT;
     }
     unsigned expired = 0;

@@ -88,27 +88,21 @@ __device__ __forceinline__ void tc_dealloc(uint32_t base, unsigned cols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr_u32(bar)) : "memory");
 }
 // 16 lanes x 16 columns: registers 4k..4k+3 = {row g, row g+8, row g (+4 columns), row g+8 (+4 columns)} of k-step k
 __device__ __forceinline__ void tc_st_16x128b_x4(uint32_t addr, const uint32_t (&r)[8]) {
   asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]));
 }
-// this lane's row, 32 columns
+// this lane's row, 32 columns; complete when the statement is (the results depend on the wait inside it)
 __device__ __forceinline__ void tc_ld_32x32b_x32(uint32_t addr, int (&r)[32]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
-      "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-        "=r"(r[31])
-      : "r"(addr)
-      : "memory");
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr));
 }
 __device__ __forceinline__ void tc_mma_i8(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -124,9 +118,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 // ---- byte expansion ------------------------------------------------------------------------------------------
 // The registers of k-steps 2q and 2q+1 for rows 16 * hl .. 16 * hl + 15 of a tile (tc_st_16x128b_x4 order).
 // Codes may keep their field's offset inside the byte (row_mult / plane shifts in `Row` undo it).
-template <int KIND> __device__ __forceinline__ void expand(const uint4 *t, int lane, int hl, int q, int plane, uint32_t (&r)[8]) {
+template <int KIND> __device__ __forceinline__ void expand(const uint4 (&t)[kind_info(KIND).chunks], int hl, int q, int plane, uint32_t (&r)[8]) {
   if constexpr (KIND == DK_TERNARY_MMA || KIND == DK_INT2_MMA) {
-    const uint4 w = t[q * 32 + lane];
+    const uint4 w = t[q];
     uint32_t m0, m1;
     if constexpr (KIND == DK_TERNARY_MMA) {
       m0 = 0x03030303u << (4 * hl);
@@ -138,12 +132,12 @@ template <int KIND> __device__ __forceinline__ void expand(const uint4 *t, int l
     r[0] = w.x & m0; r[1] = w.x & m1; r[2] = w.y & m0; r[3] = w.y & m1;
     r[4] = w.z & m0; r[5] = w.z & m1; r[6] = w.w & m0; r[7] = w.w & m1;
   } else if constexpr (KIND == LMB_INT4) {
-    const uint4 w = t[(hl * 4 + q) * 32 + lane];
+    const uint4 w = t[hl * 4 + q];
     constexpr uint32_t LO = 0x0F0F0F0Fu, HI = 0xF0F0F0F0u;
     r[0] = w.x & LO; r[1] = w.x & HI; r[2] = w.y & LO; r[3] = w.y & HI;
     r[4] = w.z & LO; r[5] = w.z & HI; r[6] = w.w & LO; r[7] = w.w & HI;
   } else if constexpr (KIND == DK_INT8_MMA) {
-    const uint4 a = t[(hl * 8 + 2 * q) * 32 + lane], b = t[(hl * 8 + 2 * q + 1) * 32 + lane];
+    const uint4 a = t[hl * 8 + 2 * q], b = t[hl * 8 + 2 * q + 1];
     r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
     r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
   } else {
@@ -154,12 +148,12 @@ template <int KIND> __device__ __forceinline__ void expand(const uint4 *t, int l
     uint32_t pa[NPL], pb[NPL];
 #pragma unroll
     for (int pl = 0; pl < NPL; ++pl) {
-      const uint4 v = t[(NC + 2 * pl + (q >> 1)) * 32 + lane];
+      const uint4 v = t[NC + 2 * pl + (q >> 1)];
       pa[pl] = (q & 1) ? v.z : v.x;
       pb[pl] = (q & 1) ? v.w : v.y;
     }
     uint4 n = make_uint4(0u, 0u, 0u, 0u);
-    if constexpr (NIB) n = t[(hl * 4 + q) * 32 + lane];
+    if constexpr (NIB) n = t[hl * 4 + q];
 #pragma unroll
     for (int kh = 0; kh < 2; ++kh)
 #pragma unroll
@@ -191,7 +185,7 @@ template <int KIND> struct Row {
 __device__ __forceinline__ int owner_of(long long u, long long total, long long g) { return int(((u + 1) * g - 1) / total); }
 
 template <int KIND, int NSMAX>
-__global__ void __launch_bounds__(bt_threads(KIND)) k_gemm_batched(const __grid_constant__ BtParams p) {
+__global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSMAX) > 1 ? 2 : 1) k_gemm_batched(const __grid_constant__ BtParams p) {
   constexpr int H = bt_halves(KIND), P = bt_planes(KIND), W = 4 * H;
   constexpr bool DD = bt_double(NSMAX);
   constexpr unsigned TB = unsigned(tile_bytes(KIND));
@@ -229,6 +223,7 @@ __global__ void __launch_bounds__(bt_threads(KIND)) k_gemm_batched(const __grid_
   const long long total = (long long)p.n_rg * p.bpr;
   const long long u0 = (long long)blockIdx.x * total / gridDim.x, u1 = (long long)(blockIdx.x + 1) * total / gridDim.x;
   const int n = int(u1 - u0);  // (row group, block) units of this CTA
+  const int rg0 = int(u0 / p.bpr), b_first = int(u0 - (long long)rg0 * p.bpr);
   const int pass = blockIdx.y;
   const unsigned img_bytes = unsigned(p.ns) * unsigned(BT_SEQ_BYTES);
   const uint8_t *img = p.img + size_t(pass) * p.bpr * img_bytes;
@@ -252,55 +247,72 @@ __global__ void __launch_bounds__(bt_threads(KIND)) k_gemm_batched(const __grid_
   };
 
   if (warp == W) {
-    if (lane == 0) {
-      int issued = 0;
-      auto weights = [&](int i) {
-        const long long u = u0 + i;
-        const int rg = int(u / p.bpr), b = int(u - (long long)rg * p.bpr), st = i % p.n_stages;
-        const BtJob &jb = p.job[job_of(rg)];
-        const int rt0 = (rg - jb.rg_first) * W, nt = min(W, jb.row_tiles - rt0);
-        uint8_t *dst = stages + size_t(st) * p.stage_bytes;
-        const uint8_t *src = jb.tiles + (size_t(rt0) * p.bpr + b) * TB;
-        int ok = nt;
-#ifdef LMB_DEBUG_BOUNDS
-        for (int k = 0; k < nt; ++k)
-          if (!LMB_IN_BOUNDS(size_t(src - jb.tiles) + size_t(k) * p.bpr * TB + TB <= jb.tiles_bytes, BOUNDS_WEIGHT_TILE, src - jb.tiles)) {
-            ok = k;
-            break;
-          }
-#endif
-        mbar_arrive_expect_tx(&full[st], unsigned(ok) * TB + img_bytes);
-        for (int k = 0; k < ok; ++k) bulk_copy_g2s(dst + k * TB, src + size_t(k) * p.bpr * TB, TB, &full[st]);
-      };
-      auto operand = [&](int i) {
-        const int b = int((u0 + i) % p.bpr), st = i % p.n_stages;
-        bulk_copy_g2s(stages + size_t(st) * p.stage_bytes + B_OFF, img + size_t(b) * img_bytes, img_bytes, &full[st]);
-      };
-      // weights do not depend on the preceding kernel, the operand images do
-      const int ahead = min(n, p.n_stages);
-      for (int i = 0; i < ahead; ++i) weights(i);
-      pdl_wait();
-      for (int i = 0; i < ahead; ++i) operand(i);
-      issued = ahead;
-      for (int i = ahead; i < n; ++i) {
-        if (!wait(&empty[i % p.n_stages], unsigned(i / p.n_stages - 1) & 1u)) break;
-        weights(i);
-        operand(i);
-        issued = i + 1;
+    // The whole warp issues: lane 0 the expected bytes, lanes 0 .. W-1 a weight tile each, lane W the operand
+    // image.  Positions advance by one unit at a time: the divisions of a flat index, per unit, held this warp
+    // below the rate of the tensor cores.
+    struct Cursor {
+      int rg, b, st;
+    };
+    auto advance = [&](Cursor &c) {
+      if (++c.b == p.bpr) {
+        c.b = 0;
+        ++c.rg;
       }
-      // own copies in flight (after a wait that expired): they land before the shared memory goes away
-      for (int i = max(0, issued - p.n_stages); i < issued; ++i)
-        for (unsigned s = 0; s < BT_DRAIN_POLLS && !mbar_try_wait(&full[i % p.n_stages], unsigned(i / p.n_stages) & 1u); ++s) {}
+      if (++c.st == p.n_stages) c.st = 0;
+    };
+    int rg_of = -1, nt = 0;
+    const uint8_t *src = nullptr;  // this lane's tile row
+    auto weights = [&](const Cursor &c) {
+      if (c.rg != rg_of) {
+        rg_of = c.rg;
+        const BtJob &jb = p.job[job_of(c.rg)];
+        const int rt0 = (c.rg - jb.rg_first) * W;
+        nt = min(W, jb.row_tiles - rt0);
+        src = jb.tiles + size_t(rt0 + lane) * p.bpr * TB;
+#ifdef LMB_DEBUG_BOUNDS
+        const size_t end = (size_t(rt0 + lane + 1) * p.bpr) * TB;
+        const bool ok = lane >= nt || LMB_IN_BOUNDS(end <= jb.tiles_bytes, BOUNDS_WEIGHT_TILE, end);
+        nt = __ffs(~__ballot_sync(0xffffffffu, ok && lane < nt)) - 1;  // a tile row that would leave its buffer is not fetched
+#endif
+      }
+      if (lane == 0) mbar_arrive_expect_tx(&full[c.st], unsigned(nt) * TB + img_bytes);
+      __syncwarp();
+      if (lane < nt) bulk_copy_g2s(stages + size_t(c.st) * p.stage_bytes + lane * TB, src + size_t(c.b) * TB, TB, &full[c.st]);
+    };
+    auto operand = [&](const Cursor &c) {
+      if (lane == W) bulk_copy_g2s(stages + size_t(c.st) * p.stage_bytes + B_OFF, img + size_t(c.b) * img_bytes, img_bytes, &full[c.st]);
+    };
+    const Cursor first{rg0, b_first, 0};
+    // weights do not depend on the preceding kernel, the operand images do
+    const int ahead = min(n, p.n_stages);
+    Cursor c = first;
+    for (int i = 0; i < ahead; ++i, advance(c)) weights(c);
+    pdl_wait();
+    Cursor o = first;
+    for (int i = 0; i < ahead; ++i, advance(o)) operand(o);
+    int issued = ahead;
+    unsigned par = 0;
+    for (int i = ahead; i < n; ++i) {
+      if (!__all_sync(0xffffffffu, wait(&empty[c.st], par))) break;
+      weights(c);
+      operand(c);
+      issued = i + 1;
+      advance(c);
+      if (c.st == 0) par ^= 1u;
     }
+    // own copies in flight (after a wait that expired): they land before the shared memory goes away
+    for (int i = max(0, issued - p.n_stages); i < issued; ++i)
+      for (unsigned s = 0; s < BT_DRAIN_POLLS && !mbar_try_wait(&full[i % p.n_stages], unsigned(i / p.n_stages) & 1u); ++s) {}
   } else if (warp == W + 1) {
     if (lane == 0) {
       const unsigned groups = unsigned(p.ns) / 2;  // 8-row groups of B: two sequences x four digits
       const uint32_t idesc = (2u << 4) | (KIND == DK_INT8_MMA ? 1u << 7 : 0u) | (1u << 10) | ((unsigned(p.ns) * 4u >> 3) << 17) | (8u << 24);
       const uint64_t lbo = groups * 128u >> 4, sbo = 128u >> 4;  // core matrices: [16-column chunk][8-row group][8 rows][16 bytes]
       bool ok = true;
+      int st = 0;
+      unsigned st_par = 0;
       for (int i = 0; i < n && ok; ++i) {
-        const int st = i % p.n_stages;
-        ok = wait(&full[st], unsigned(i / p.n_stages) & 1u);
+        ok = wait(&full[st], st_par);
         const uint64_t bdesc0 = (uint64_t(1) << 46) | (sbo << 32) | (lbo << 16) |
                                 uint64_t((smem_addr_u32(stages) + unsigned(st) * p.stage_bytes + B_OFF) >> 4);
         for (int pl = 0; pl < P && ok; ++pl) {
@@ -314,6 +326,10 @@ __global__ void __launch_bounds__(bt_threads(KIND)) k_gemm_batched(const __grid_
             for (int s = 0; s < 8; ++s) tc_mma_i8(d, a + 8 * s, bdesc0 + uint64_t(2 * s) * lbo, idesc, s > 0);
             tc_commit(&d_full[h][buf]);
           }
+        }
+        if (++st == p.n_stages) {
+          st = 0;
+          st_par ^= 1u;
         }
       }
       // no MMA is in flight when the TMEM is given back, whatever the workers have waited for
@@ -331,8 +347,7 @@ __global__ void __launch_bounds__(bt_threads(KIND)) k_gemm_batched(const __grid_
     const int nb = min(p.ns, p.batch - pass * p.ns);
 
     // finished row group (or this CTA's part of it)
-    auto flush = [&](long long u) {
-      const int rg = int(u / p.bpr);
+    auto flush = [&](int rg) {
       const BtJob &jb = p.job[job_of(rg)];
       const int rt = (rg - jb.rg_first) * W + warp, row = rt * TILE_ROWS + lane;
       float v[NSMAX];
@@ -415,8 +430,9 @@ __global__ void __launch_bounds__(bt_threads(KIND)) k_gemm_batched(const __grid_
     };
 
     // accumulator of unit u (block i = u / P) -> fp32
-    auto readout = [&](int u) -> bool {
-      const int i = u / P, plane = u % P, st = i % p.n_stages, buf = u & 1;
+    int rg = rg0, b = b_first, st_r = 0;  // where the read-out stands
+    auto readout = [&](int u, bool last_unit) -> bool {
+      const int plane = u % P, st = st_r, buf = u & 1;
       if (!__all_sync(0xffffffffu, wait(&d_full[h][buf], unsigned(u >> 1) & 1u))) return false;
       tc_fence_after();
       const uint8_t *stage = stages + size_t(st) * p.stage_bytes;
@@ -431,7 +447,6 @@ __global__ void __launch_bounds__(bt_threads(KIND)) k_gemm_batched(const __grid_
         if (q0 < p.ns) {
           int r[32];
           tc_ld_32x32b_x32(d + 4 * q0, r);
-          tc_wait_ld();
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const int4 ax = aux[q0 + q];  // {block scale, digit-pair sums}; beyond p.ns: unused columns
@@ -452,18 +467,31 @@ __global__ void __launch_bounds__(bt_threads(KIND)) k_gemm_batched(const __grid_
       if (plane == P - 1) {
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[st]);
-        const long long ug = u0 + i;
-        if (i + 1 == n || (ug + 1) % p.bpr == 0) flush(ug);
+        if (++st_r == p.n_stages) st_r = 0;
+        const bool row_end = ++b == p.bpr;
+        if (last_unit || row_end) flush(rg);
+        if (row_end) {
+          b = 0;
+          ++rg;
+        }
       }
       return true;
     };
 
     bool ok = true;
+    int st_w = 0;
+    unsigned par_w = 0;
     for (int i = 0; i < n && ok; ++i) {
-      const int st = i % p.n_stages;
-      ok = __all_sync(0xffffffffu, wait(&full[st], unsigned(i / p.n_stages) & 1u));
+      ok = __all_sync(0xffffffffu, wait(&full[st_w], par_w));
       if (!ok) break;
-      const uint4 *tile = reinterpret_cast<const uint4 *>(stages + size_t(st) * p.stage_bytes + warp * TB);
+      const uint4 *tile = reinterpret_cast<const uint4 *>(stages + size_t(st_w) * p.stage_bytes + warp * TB);
+      uint4 raw[kind_info(KIND).chunks];
+#pragma unroll
+      for (int k = 0; k < kind_info(KIND).chunks; ++k) raw[k] = tile[k * 32 + lane];
+      if (++st_w == p.n_stages) {
+        st_w = 0;
+        par_w ^= 1u;
+      }
 #pragma unroll
       for (int pl = 0; pl < P; ++pl) {
         const int u = i * P + pl, buf = u & 1;
@@ -474,21 +502,21 @@ __global__ void __launch_bounds__(bt_threads(KIND)) k_gemm_batched(const __grid_
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             uint32_t r[8];
-            expand<KIND>(tile, lane, hl, q, pl, r);
+            expand<KIND>(raw, hl, q, pl, r);
             tc_st_16x128b_x4(a + (uint32_t(hl) << 20) + 16 * q, r);
           }
         tc_wait_st();
         // one accumulator: its last unit is read before the next MMAs are let go
-        if (!DD && u > 0) ok = readout(u - 1);
+        if (!DD && u > 0) ok = readout(u - 1, false);
         if (!ok) break;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&a_full[h][buf]);
-        if (DD && u > 0) ok = readout(u - 1);
+        if (DD && u > 0) ok = readout(u - 1, false);
         if (!ok) break;
       }
     }
-    if (ok && n > 0) readout(n * P - 1);
+    if (ok && n > 0) readout(n * P - 1, true);
   }
   __syncwarp();
   tc_fence_before();

@@ -5,6 +5,8 @@ import pytest
 
 from lutmac_b200 import _lib, api, synth
 from lutmac_b200.blocks import BINARY, INT2, INT3, INT4, INT5, INT6, INT8, TERNARY, blocks_per_row
+from lutmac_b200.model import Model
+from oracle.oracle import OracleModel
 from tests.conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +67,22 @@ def test_batched_expired_wait_is_reported(ctx):
     finally:
         _lib.check(L.lmb_debug_batched_waits(ctx.h, 0, 0))
     assert np.array_equal(api.lut_linear(t, None, x, None, 4, ctx=ctx), want)
+
+
+@pytest.mark.parametrize("head_dim,n_heads,n_kv", [(64, 8, 2), (64, 6, 1), (128, 4, 2)])
+def test_batched_attention_positions(ctx, oracle, head_dim, n_heads, n_kv):
+    """The streaming attention form: chunk edges (32 and 64 positions), sequences at different positions, an empty
+    cache, splits without positions; every sequence against the oracle's own decode."""
+    shape = dict(synth.tiny_model_shape(), head_dim=head_dim, n_heads=n_heads, n_kv_heads=n_kv, n_layers=1)
+    spec = synth.model_spec(shape, INT4, seed=3, max_seq=160)
+    m = Model(spec, ctx, max_batch=3)
+    refs = [OracleModel(oracle, spec) for _ in range(3)]
+    rng = np.random.default_rng(8)
+    for p in range(131):
+        toks, pos = rng.integers(0, spec.cfg["vocab"], size=3), [p, p // 2, p // 5]
+        got = m.forward(toks.astype(np.int32), pos)
+        for q in range(3):
+            want = refs[q].forward(int(toks[q]), pos[q])
+            if p in (0, 1, 31, 32, 33, 63, 64, 65, 66, 127, 128, 130):
+                assert rel_l2(got[q], want) < 1e-5, (p, q)
+    m.close()

@@ -15,7 +15,10 @@
 // operand loads and the scaling of every (32 rows x 2 sequences) in the same warps; here the weights are
 // read once per 32 sequences and the tensor work leaves the warps, which keep the byte expansion
 // (64 masks per 32 x 256 codes) and the scaling (9 instructions per row, sequence and block).  Ternary
-// 8192 x 28672, 16 sequences: 133 us before, 45 us with this kernel (9.9 us of HBM time).
+// 8192 x 28672, 16 sequences: 133 us before, 44 us with this kernel (9.9 us of HBM time).  Measured on the way
+// and not taken: two warps per tile (46 us; 24 instead of 19 us at 8192 x 8192).  With an eighth of the MMAs,
+// of the scaling or of the TMEM stores it takes 38 to 43 us, with an eighth of all three 27 us, with an eighth
+// of the bytes 42 us: what is left is the chain of expansion, hand-over and scaling inside a warp.
 //
 // Work split: the (row group, block) units of all jobs of a launch are one flat list, cut into equal
 // contiguous ranges, one per CTA, whatever the shapes: no nearly empty last wave.  A row group whose
@@ -341,9 +344,24 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
     const int h = warp >> 2;
     const uint32_t lanes = uint32_t(warp & 3) << 21;  // this warp's 32 TMEM lanes
     const int m = lane >> 3, sc_at = 4 * (lane & 7) + m;
+    // low and high digit pairs of up to 8 blocks, and the sum of what they were before: two levels keep the fp32
+    // error of a long row below that of the short slices a single-sequence launch cuts it into
     float2 acc[NSMAX];
+    float sum[NSMAX];
 #pragma unroll
-    for (int q = 0; q < NSMAX; ++q) acc[q] = make_float2(0.0f, 0.0f);
+    for (int q = 0; q < NSMAX; ++q) {
+      acc[q] = make_float2(0.0f, 0.0f);
+      sum[q] = 0.0f;
+    }
+    int in_acc = 0;
+    auto fold = [&]() {
+#pragma unroll
+      for (int q = 0; q < NSMAX; ++q) {
+        sum[q] += acc[q].x + 65536.0f * acc[q].y;
+        acc[q] = make_float2(0.0f, 0.0f);
+      }
+      in_acc = 0;
+    };
     const int nb = min(p.ns, p.batch - pass * p.ns);
 
     // finished row group (or this CTA's part of it)
@@ -353,8 +371,8 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
       float v[NSMAX];
 #pragma unroll
       for (int q = 0; q < NSMAX; ++q) {
-        v[q] = acc[q].x + 65536.0f * acc[q].y;
-        acc[q] = make_float2(0.0f, 0.0f);
+        v[q] = sum[q];
+        sum[q] = 0.0f;
       }
       if (rt >= jb.row_tiles) return;  // uniform over the warp
       const int c0 = owner_of((long long)rg * p.bpr, total, gridDim.x), c1 = owner_of((long long)rg * p.bpr + p.bpr - 1, total, gridDim.x);
@@ -469,6 +487,7 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
         if (lane == 0) mbar_arrive(&empty[st]);
         if (++st_r == p.n_stages) st_r = 0;
         const bool row_end = ++b == p.bpr;
+        if (++in_acc == 8 || last_unit || row_end) fold();
         if (last_unit || row_end) flush(rg);
         if (row_end) {
           b = 0;
@@ -731,7 +750,6 @@ int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate,
   LMB_CUDA(cudaLaunchKernelEx(&cfg, k_prepare_batched, args[0].x, args[0].x2, unsigned(args[0].x_len), unsigned(args[0].x_stride), p.bpr, xmode,
                               rotate ? 1 : 0, eps, p.ns, reinterpret_cast<uint8_t *>(ctx->xprep)));
   ctx->launches++;
-  ctx->fault_unread = true;
   switch (kind) {
   case LMB_INT4: return launch_kind<LMB_INT4>(ctx, p, pl);
   case DK_TERNARY_MMA: return launch_kind<DK_TERNARY_MMA>(ctx, p, pl);

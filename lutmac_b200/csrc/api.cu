@@ -49,20 +49,15 @@ int ensure_scratch(lmb_ctx *ctx, size_t floats, size_t counters) {
 
 // A launch that left early may have left arrival counters behind: they start from zero again.
 int clear_fault(lmb_ctx *ctx) {
-  LMB_CUDA(cudaMemsetAsync(ctx->d_fault, 0, sizeof(unsigned), ctx->stream));
+  *ctx->fault = 0u;
   LMB_CUDA(cudaMemsetAsync(ctx->counters, 0, ctx->n_counters * sizeof(unsigned), ctx->stream));
   LMB_CUDA(cudaStreamSynchronize(ctx->stream));
   return LMB_OK;
 }
 
-// After the stream has been waited for: LMB_ERR_TIMEOUT if a batched launch gave up a bounded wait.
+// After the stream has been waited for: LMB_ERR_TIMEOUT if a launch gave up a bounded wait.
 int check_fault(lmb_ctx *ctx, const char *who) {
-  if (!ctx->fault_unread || !ctx->d_fault) return LMB_OK;
-  unsigned v = 0;
-  LMB_CUDA(cudaMemcpyAsync(&v, ctx->d_fault, sizeof v, cudaMemcpyDeviceToHost, ctx->stream));
-  LMB_CUDA(cudaStreamSynchronize(ctx->stream));
-  ctx->fault_unread = false;
-  if (!v) return LMB_OK;
+  if (!ctx->fault || *ctx->fault == 0u) return LMB_OK;
   int st = clear_fault(ctx);
   if (st != LMB_OK) return st;
   set_last_error(std::string(who) + ": a bounded wait for asynchronous copies expired in a kernel");
@@ -266,8 +261,13 @@ int lmb_ctx_create(int device, lmb_ctx **out) {
   int st = configure_gemv(ctx);
   if (st == LMB_OK) st = ensure_scratch(ctx, size_t(4) << 20, size_t(1) << 16);
   if (st == LMB_OK) {
-    e = cudaMalloc(&ctx->d_fault, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(ctx->d_fault, 0, sizeof(unsigned));
+    void *flag = nullptr;
+    e = cudaHostAlloc(&flag, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e == cudaSuccess) {
+      ctx->fault = static_cast<volatile unsigned *>(flag);
+      *ctx->fault = 0u;
+      e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&ctx->d_fault), flag, 0);
+    }
     if (e != cudaSuccess) st = cuda_fail(e, "lmb_ctx_create");
   }
   if (st != LMB_OK) {
@@ -338,7 +338,7 @@ int lmb_ctx_destroy(lmb_ctx *ctx) {
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->counters) cudaFree(ctx->counters);
   if (ctx->xprep) cudaFree(ctx->xprep);
-  if (ctx->d_fault) cudaFree(ctx->d_fault);
+  if (ctx->fault) cudaFreeHost(const_cast<unsigned *>(ctx->fault));
   if (ctx->d_timeline) cudaFree(ctx->d_timeline);
   if (ctx->h_upload) cudaFreeHost(ctx->h_upload);
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -632,7 +632,7 @@ int lmb_linear_host(lmb_ctx *ctx, const lmb_weight *w, const float *bias, const 
   LMB_REQUIRE(ctx && w && input && output && batch > 0, "lmb_linear_host: null argument");
   const size_t K = w->K, M = w->M;
   const size_t in_f = batch * K, out_f = batch * M, bias_f = bias ? M : 0;
-  int st = ensure_stage(ctx, (in_f + out_f + bias_f + 1) * sizeof(float));
+  int st = ensure_stage(ctx, (in_f + out_f + bias_f) * sizeof(float));
   if (st != LMB_OK) return st;
   float *h = static_cast<float *>(ctx->h_stage), *d = ctx->d_stage;
   std::memcpy(h, input, in_f * sizeof(float));
@@ -643,13 +643,7 @@ int lmb_linear_host(lmb_ctx *ctx, const lmb_weight *w, const float *bias, const 
   if (st != LMB_OK) return st;
   float *h_y = h + in_f + bias_f;
   LMB_CUDA(cudaMemcpyAsync(h_y, d_y, out_f * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-  // the fault flag of a batched launch rides behind the outputs
-  unsigned *h_fault = reinterpret_cast<unsigned *>(h_y + out_f);
-  const bool look = ctx->fault_unread;
-  *h_fault = 0;
-  if (look) LMB_CUDA(cudaMemcpyAsync(h_fault, ctx->d_fault, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
   LMB_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (look && *h_fault == 0) ctx->fault_unread = false;
   std::memcpy(output, h_y, out_f * sizeof(float));
   return check_fault(ctx, "lmb_linear_host");
 }

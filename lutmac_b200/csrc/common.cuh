@@ -189,11 +189,12 @@ struct lmb_ctx {
   // activations prepared once per launch for batched GEMVs (digits, block scales, digit sums)
   uint32_t *xprep = nullptr;
   size_t xprep_blocks = 0;  // capacity in (sequence, block) pairs
-  // set by a kernel whose bounded wait (for its own asynchronous copies) ran out; read with the logits
+  // set by a kernel whose bounded wait (for its own asynchronous copies) ran out.  Page-locked host memory that
+  // kernels write only then, so that looking at it after a synchronisation costs no copy (2 to 5 us each).
   unsigned *d_fault = nullptr;
   unsigned batched_spin_limit = 1u << 22;  // polls before a wait of the batched kernel gives up (seconds)
   int batched_extra_arrivals = 0;          // test hook, lmb_debug_batched_waits
-  bool fault_unread = false;  // a batched launch may have set it since it was last read (lmb_ctx_sync, host entry points)
+  volatile unsigned *fault = nullptr;  // the flag as the host sees it
   // launch timeline (debugging, lmb_debug_launch_timeline): 8 time stamps per launch, null when off
   unsigned long long *d_timeline = nullptr;
   int timeline_cap = 0, timeline_cursor = 0, timeline_used = 0;  // used: most slots any step has taken (graph replays launch nothing)

@@ -834,17 +834,16 @@ int lmb_model_forward(lmb_model *m, const int *token_ids, const size_t *position
   }
 fetch:
   if (h_logits) {
-    // the logits and, behind them in the same stream, the three status words a step can leave: the
-    // context's fault flag, the exchange block's time-out flag, the persistent step's status
+    // the logits and, behind them in the same stream, the status words a step can leave: the exchange
+    // block's time-out flag, the persistent step's status; the context's fault flag is host memory
     unsigned *hs = static_cast<unsigned *>(m->h_status);
     hs[0] = hs[1] = 0;
     LMB_CUDA(cudaMemcpyAsync(h_logits, m->logits, batch * c.vocab_size * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    LMB_CUDA(cudaMemcpyAsync(&hs[0], ctx->d_fault, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     if (c.tp_size > 1 && ctx->xchg.ready)
       LMB_CUDA(cudaMemcpyAsync(&hs[1], &static_cast<XchgHeader *>(ctx->xchg.local)->timed_out, sizeof(unsigned),
                                cudaMemcpyDeviceToHost, ctx->stream));
     LMB_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (hs[0]) {  // a kernel's bounded wait for its own asynchronous copies ran out
+    if (*ctx->fault) {  // a kernel's bounded wait for its own asynchronous copies ran out
       st = clear_fault(ctx);
       if (st != LMB_OK) return st;
       set_last_error("lmb_model_forward: a bounded wait for asynchronous copies expired in the attention kernel or a batched projection");

@@ -133,7 +133,8 @@ __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn_group(const AttnArg
 // and with many waves of short slices paid its set-up and merge 37 times per KV head.  Here queries and
 // sums live in registers, a key or value row is read once for all heads, and the 32 partial dot products
 // of a lane are reduced together (31 shuffles for 32 sums).
-// Measured, 16 sequences at 2040 positions, 8 KV heads of 8 queries x 128: ATTN_BEFORE us before, ATTN_AFTER us now (41 us of HBM time).
+// Measured, 16 sequences at 2040 positions, 8 KV heads of 8 queries x 128: 130 us before; the 4-layer step it is part of went from
+// 1.35 to 1.02 ms a token (41 us of HBM time a layer).
 constexpr int STREAM_STAGES = 3;
 constexpr int STREAM_THREADS = 256;
 constexpr int STREAM_WARPS = STREAM_THREADS / 32;

@@ -169,6 +169,10 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
       if (sub + sl * wpr < ns && tile_ok(row_tiles + size_t(sub + sl * wpr) * TB)) slot[sl].load(row_tiles + size_t(sub + sl * wpr) * TB, lane);
   }
 
+  // so is the norm weight of the first block this warp converts
+  float w8[8];
+  if (NSEQ == 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered && warp < ns) load_x8(job.x2, job.x_len, size_t(b0 + warp), lane, w8);
+
   pdl_wait();
   if (threadIdx.x == 0) {
     tl_min(p.dbg, 1);
@@ -179,8 +183,13 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
   const unsigned epoch = p.peer.n ? *reinterpret_cast<volatile unsigned *>(p.peer.epoch) : 0u;
   const float *x = job.x + size_t(batch0) * job.x_stride;
   float *inv_rms = part[0];  // [sequence] after the block below (XMODE_RMSNORM)
-  if (p.xmode == XMODE_RMSNORM && !p.prep && !clustered) {
-    // RMSNorm of the whole input vectors (src/layers/norm.cpp:18-34), recomputed by every CTA
+  // One sequence: RMSNorm (src/layers/norm.cpp:18-34) is linear in 1 / rms, so the digits below are those of
+  // x * w and the row sums are multiplied by 1 / rms at the end: the sum of squares and the conversion read x
+  // side by side, instead of one round trip and two barriers after the other (1B-shaped step with the
+  // page-locked logits: 611 -> 558 us).
+  const bool late_rms = NSEQ == 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered;
+  if (NSEQ > 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered) {
+    // RMSNorm of the whole input vectors, recomputed by every CTA
     float ss[NSEQ];
 #pragma unroll
     for (int q = 0; q < NSEQ; ++q) ss[q] = 0.0f;
@@ -246,7 +255,7 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
       // cluster (which covers all of K), and the block scales are multiplied by 1 / rms afterwards.
       const int Cr = p.cl_size / job.n_ks, cr = crank / job.n_ks;
       const int mine = ns > cr ? (ns - cr + Cr - 1) / Cr : 0;
-      float v[8], w8[8], nv[8];
+      float v[8], nv[8];
       if (warp < mine) load_x8(x, job.x_len, size_t(b0 + cr + warp * Cr), lane, nv);
       for (int it = warp; it < mine; it += WARPS) {
         const int bl = cr + it * Cr;
@@ -308,21 +317,32 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
   }
   if (!(kind_is_mma(KIND) && p.prep) && !clustered) {
     // one warp per (sequence, block); the next item's activations are fetched while this one is converted
-    float v[8], w8[8], nv[8];
+    float v[8], nv[8];
     const int items = ns * nb;
+    auto second = [&](int q, int bl) {  // norm weight, or the vector multiplied in
+      if (p.xmode == XMODE_RMSNORM) load_x8(job.x2, job.x_len, size_t(b0 + bl), lane, w8);
+      if (p.xmode == XMODE_SILU_MUL || p.xmode == XMODE_GELU_MUL) load_x8(job.x2 + size_t(batch0 + q) * job.x_stride, job.x_len, size_t(b0 + bl), lane, w8);
+    };
     if (warp < items) load_x8(x + size_t(NSEQ == 1 ? 0 : warp / ns) * job.x_stride, job.x_len, size_t(b0 + (NSEQ == 1 ? warp : warp % ns)), lane, nv);
+    if (late_rms) {
+      float ss = 0.0f;
+#pragma unroll 8
+      for (unsigned i = threadIdx.x; i < job.x_len; i += THREADS) ss += x[i] * x[i];
+#pragma unroll
+      for (int m = 16; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+      if (lane == 0) xsum[64 - WARPS + warp] = ss;  // a slice has at most 48 blocks
+    }
     for (int it = warp; it < items; it += WARPS) {
       const int q = NSEQ == 1 ? 0 : it / ns, bl = it - q * ns;
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = nv[e];
-      if (p.xmode == XMODE_RMSNORM) load_x8(job.x2, job.x_len, size_t(b0 + bl), lane, w8);
-      if (p.xmode == XMODE_SILU_MUL || p.xmode == XMODE_GELU_MUL) load_x8(job.x2 + size_t(batch0 + q) * job.x_stride, job.x_len, size_t(b0 + bl), lane, w8);
+      if (!late_rms || it != warp) second(q, bl);
       if (it + WARPS < items) {
         const int nq = NSEQ == 1 ? 0 : (it + WARPS) / ns;
         load_x8(x + size_t(nq) * job.x_stride, job.x_len, size_t(b0 + (it + WARPS) - nq * ns), lane, nv);
       }
       if (p.xmode == XMODE_RMSNORM) {
-        const float ir = inv_rms[q];
+        const float ir = late_rms ? 1.0f : inv_rms[q];
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = v[e] * ir * w8[e];
       } else if (p.xmode == XMODE_SILU_MUL) {
@@ -387,7 +407,7 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
 
   // combine the warps that share a row-tile, in warp order: thread t ends up with row rt0*32 + t
   if (threadIdx.x == 0) tl_max(p.dbg, 4);
-  if (p.xmode == XMODE_RMSNORM && !p.prep && !clustered) __syncthreads();  // inv_rms (in part[0]) has been read by everyone
+  if (NSEQ > 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered) __syncthreads();  // inv_rms (in part[0]) has been read by everyone
 #pragma unroll
   for (int q = 0; q < NSEQ; ++q) part[q][threadIdx.x] = acc[q];
   __syncthreads();
@@ -401,6 +421,12 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
       const int r = t >> 5;
       for (int k = 0; k < wpr; ++k) s[q] += part[q][(r * wpr + k) * 32 + (t & 31)];
     }
+  }
+  if (late_rms) {
+    float tot = 0.0f;
+#pragma unroll
+    for (int k = 0; k < WARPS; ++k) tot += xsum[64 - WARPS + k];
+    s[0] *= 1.0f / sqrtf(tot / float(job.x_len) + p.eps);
   }
   const int row = rt0 * TILE_ROWS + t;
   // one output element; with tensor parallelism it goes to this rank's slot in every rank's block

@@ -228,6 +228,10 @@ int lmb_debug_force_plan(int R, int n_ks, int cr);
 /* Tests: from now on the batched projections' operand barriers expect `extra_arrivals` arrivals too many
  * and their waits give up after `spin_limit` polls (0: the default); 0, 0: off. */
 int lmb_debug_batched_waits(lmb_ctx *ctx, int extra_arrivals, unsigned spin_limit);
+/* Tests: from now on the attention launches of several sequences cut the cache into `n_splits` parts, the
+ * barriers that hand a ring stage back expect `extra_arrivals` arrivals too many, and waits give up after
+ * `spin_limit` polls (0: the defaults).  Steps captured into graphs earlier keep what they were captured with. */
+int lmb_debug_attn_stream(lmb_ctx *ctx, int n_splits, int extra_arrivals, unsigned spin_limit);
 /* Range-checking build (liblutmac_b200_dbg.so, compiled with -DLMB_DEBUG_BOUNDS; the reference has no
  * sanitizer set-up to mirror): the GEMV kernels check every weight-tile load, output store and
  * split-K scratch store against the extent of its buffer, the attention kernel its cache slices; an

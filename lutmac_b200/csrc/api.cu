@@ -47,9 +47,11 @@ int ensure_scratch(lmb_ctx *ctx, size_t floats, size_t counters) {
   return LMB_OK;
 }
 
-// A launch that left early may have left arrival counters behind: they start from zero again.
+// A launch that left early may have left arrival counters behind: the context's start from zero again here, a
+// model's before its next step (fault_gen), whichever call it was that reported the fault.
 int clear_fault(lmb_ctx *ctx) {
   *ctx->fault = 0u;
+  ctx->fault_gen++;
   LMB_CUDA(cudaMemsetAsync(ctx->counters, 0, ctx->n_counters * sizeof(unsigned), ctx->stream));
   LMB_CUDA(cudaStreamSynchronize(ctx->stream));
   return LMB_OK;

@@ -195,6 +195,10 @@ struct lmb_ctx {
   unsigned batched_spin_limit = 1u << 22;  // polls before a wait of the batched kernel gives up (seconds)
   int batched_extra_arrivals = 0;          // test hook, lmb_debug_batched_waits
   volatile unsigned *fault = nullptr;  // the flag as the host sees it
+  uint64_t fault_gen = 0;              // faults reported so far: models clear their own arrival counters when it has moved
+  // test hook, lmb_debug_attn_stream
+  int attn_force_splits = 0, attn_extra_arrivals = 0;
+  unsigned attn_spin_limit = 0;
   // launch timeline (debugging, lmb_debug_launch_timeline): 8 time stamps per launch, null when off
   unsigned long long *d_timeline = nullptr;
   int timeline_cap = 0, timeline_cursor = 0, timeline_used = 0;  // used: most slots any step has taken (graph replays launch nothing)

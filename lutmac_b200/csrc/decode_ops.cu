@@ -145,7 +145,8 @@ template <int PER> __host__ __device__ constexpr size_t stream_smem_floats() {
 }
 
 template <int PER, int G>
-__global__ void __launch_bounds__(STREAM_THREADS, 2) k_decode_attn_stream(const AttnArgs a, const RopeDims d, unsigned spin_limit, unsigned *timed_out) {
+__global__ void __launch_bounds__(STREAM_THREADS, 2) k_decode_attn_stream(const AttnArgs a, const RopeDims d, unsigned spin_limit, int extra_arrivals,
+                                                                          unsigned *timed_out) {
   constexpr int T = 32 / G, HD = 32 * PER, CH = stream_chunk<PER>(), ST = STREAM_STAGES;
   static_assert(CH % (STREAM_WARPS * T) == 0, "whole rounds");
   extern __shared__ __align__(128) float sm[];
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_decode_attn_stream(const 
     gave_up = 0;
     for (int s = 0; s < ST; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], STREAM_WARPS);
+      mbar_init(&empty[s], unsigned(STREAM_WARPS + extra_arrivals));
     }
   }
   __syncthreads();
@@ -595,13 +596,15 @@ int launch_decode_attn_group(lmb_ctx *ctx, const float *q, const float *k, const
     if (plan.per == 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_group<4, true>, a, d, ctx->xchg.spin_limit, flag, tl));
     else LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_group<2, true>, a, d, ctx->xchg.spin_limit, flag, tl));
   } else {
-    a.n_splits = stream_splits(d.nkv, batch, d.max_seq, size_t(ctx->sm_count));
+    a.n_splits = ctx->attn_force_splits ? ctx->attn_force_splits : stream_splits(d.nkv, batch, d.max_seq, size_t(ctx->sm_count));
+    const unsigned limit = ctx->attn_spin_limit ? ctx->attn_spin_limit : ctx->xchg.spin_limit;
+    const int extra = ctx->attn_extra_arrivals;
     cfg.gridDim = dim3(unsigned(d.nkv * size_t(a.n_splits)), unsigned(batch));
     cfg.dynamicSmemBytes = (plan.per == 4 ? stream_smem_floats<4>() : stream_smem_floats<2>()) * sizeof(float);
     // four query heads per KV head or fewer: eight positions per round instead of four
-    if (plan.per == 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<4, 8>, a, d, ctx->xchg.spin_limit, flag));
-    else if (d.nh / d.nkv > 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<2, 8>, a, d, ctx->xchg.spin_limit, flag));
-    else LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<2, 4>, a, d, ctx->xchg.spin_limit, flag));
+    if (plan.per == 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<4, 8>, a, d, limit, extra, flag));
+    else if (d.nh / d.nkv > 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<2, 8>, a, d, limit, extra, flag));
+    else LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<2, 4>, a, d, limit, extra, flag));
   }
   ctx->launches++;
   return LMB_OK;
@@ -633,3 +636,11 @@ int configure_decode_ops(lmb_ctx *ctx) {
 }
 
 }  // namespace lmb
+
+extern "C" int lmb_debug_attn_stream(lmb_ctx *ctx, int n_splits, int extra_arrivals, unsigned spin_limit) {
+  LMB_REQUIRE(ctx && n_splits >= 0 && n_splits <= lmb::ATT_MAX_SPLITS && extra_arrivals >= 0, "lmb_debug_attn_stream: bad argument");
+  ctx->attn_force_splits = n_splits;
+  ctx->attn_extra_arrivals = extra_arrivals;
+  ctx->attn_spin_limit = spin_limit;
+  return LMB_OK;
+}

@@ -294,6 +294,7 @@ int lmb_model_create(lmb_ctx *ctx, const lmb_model_config *c, lmb_model **out) {
   lmb_model *m = new (std::nothrow) lmb_model();
   if (!m) return LMB_ERR_ALLOC;
   m->ctx = ctx;
+  m->fault_gen = ctx->fault_gen;
   m->cfg = *c;
   m->cfg.tp_size = g;
   m->nh = c->num_attention_heads / g;
@@ -626,6 +627,11 @@ int lmb_model_forward(lmb_model *m, const int *token_ids, const size_t *position
   size_t *hp = reinterpret_cast<size_t *>(static_cast<char *>(m->h_io) + c.max_batch * sizeof(int));
   if (!m->capturing) {
     LMB_CUDA(cudaStreamSynchronize(ctx->stream));  // the staging buffer may still be in use by the previous step
+    if (m->fault_gen != ctx->fault_gen) {
+      // a split that gave up its wait never arrived, others may have: the counters start from zero again
+      LMB_CUDA(cudaMemsetAsync(m->att_counters, 0, c.max_batch * m->nh * sizeof(unsigned), ctx->stream));
+      m->fault_gen = ctx->fault_gen;
+    }
     std::memcpy(ht, token_ids, batch * sizeof(int));
     std::memcpy(hp, positions, batch * sizeof(size_t));
     LMB_CUDA(cudaMemcpyAsync(m->d_tokens, ht, batch * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
@@ -853,6 +859,7 @@ fetch:
     int ps = persist_take_status(m, &expired);
     if (ps != LMB_OK) return ps;
     if (expired) {
+      ctx->fault_gen++;  // phases after the one that expired did not run to their end: see above
       set_last_error("lmb_model_forward: a bounded wait between the phases of the decode step expired (phase " +
                      std::to_string(expired - 1) + ")");
       return LMB_ERR_TIMEOUT;

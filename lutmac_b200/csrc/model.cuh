@@ -29,6 +29,7 @@ struct lmb_model {
         *gate = nullptr, *up = nullptr, *act = nullptr, *logits = nullptr, *logits_local = nullptr, *logits_gather = nullptr;
   float *att_partial = nullptr;      // [max_batch][nh][32 splits][hd + 2]
   unsigned *att_counters = nullptr;  // [max_batch][nh]
+  uint64_t fault_gen = 0;            // lmb_ctx::fault_gen when att_counters were last known to be zero between steps
   float *kv = nullptr;        // [max_batch][L][2][nkv][max_seq][hd]: the positions of one head contiguous
   float *cs_table = nullptr;  // [max_seq][hd/2 cos | hd/2 sin]
   int *d_tokens = nullptr;

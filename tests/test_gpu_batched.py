@@ -86,3 +86,40 @@ def test_batched_attention_positions(ctx, oracle, head_dim, n_heads, n_kv):
             if p in (0, 1, 31, 32, 33, 63, 64, 65, 66, 127, 128, 130):
                 assert rel_l2(got[q], want) < 1e-5, (p, q)
     m.close()
+
+
+def _models_with_context(ctx, oracle, head_dim, n_heads, n_kv, positions, seed):
+    """A one-layer model and one oracle per sequence, all holding the same random cache."""
+    shape = dict(synth.tiny_model_shape(), head_dim=head_dim, n_heads=n_heads, n_kv_heads=n_kv, n_layers=1)
+    spec = synth.model_spec(shape, INT4, seed=seed, max_seq=max(positions) + 8)
+    m = Model(spec, ctx, max_batch=len(positions))
+    refs = [OracleModel(oracle, spec) for _ in positions]
+    rng = np.random.default_rng(seed)
+    for q, ref in enumerate(refs):
+        ref.kv[...] = rng.standard_normal(ref.kv.shape).astype(np.float32)
+        m.kv_import(ref.kv, q)
+    return spec, m, refs, rng
+
+
+@pytest.mark.parametrize("head_dim,pos", [(64, 385), (128, 193)])
+def test_step_after_an_expired_attention_wait(ctx, oracle, head_dim, pos, monkeypatch):
+    """Two splits, of which the first has one chunk more than the ring has stages and the second has not: with
+    a refill barrier that never completes the first leaves without arriving, the second arrives.  The step
+    reports it, and the following steps (other tokens) are right."""
+    monkeypatch.setenv("LMB_MODEL_GRAPH", "0")
+    L = _lib.lib()
+    spec, m, refs, rng = _models_with_context(ctx, oracle, head_dim, 4, 2, [pos, pos], 17)
+    toks = rng.integers(0, spec.cfg["vocab"], size=(4, 2)).astype(np.int32)
+    try:
+        _lib.check(L.lmb_debug_attn_stream(ctx.h, 2, 1, 2000))
+        with pytest.raises(_lib.LutmacError) as e:
+            m.forward(toks[0], [pos, pos])
+        assert e.value.status == _lib.ERR_TIMEOUT
+        _lib.check(L.lmb_debug_attn_stream(ctx.h, 2, 0, 0))
+        for s in range(1, 4):
+            got = m.forward(toks[s], [pos + s - 1] * 2)
+            for q in range(2):
+                assert rel_l2(got[q], refs[q].forward(int(toks[s][q]), pos + s - 1)) < 1e-5, (s, q)
+    finally:
+        _lib.check(L.lmb_debug_attn_stream(ctx.h, 0, 0, 0))
+    m.close()

@@ -307,6 +307,9 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
     for (int i = max(0, issued - p.n_stages); i < issued; ++i)
       for (unsigned s = 0; s < BT_DRAIN_POLLS && !mbar_try_wait(&full[i % p.n_stages], unsigned(i / p.n_stages) & 1u); ++s) {}
   } else if (warp == W + 1) {
+    // Nothing to do before the operand copies, which wait for the preceding kernels: polling earlier would charge
+    // those kernels' run time (another rank's lateness among it) to this kernel's limit.
+    pdl_wait();
     if (lane == 0) {
       const unsigned groups = unsigned(p.ns) / 2;  // 8-row groups of B: two sequences x four digits
       const uint32_t idesc = (2u << 4) | (KIND == DK_INT8_MMA ? 1u << 7 : 0u) | (1u << 10) | ((unsigned(p.ns) * 4u >> 3) << 17) | (8u << 24);

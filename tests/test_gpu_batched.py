@@ -69,6 +69,31 @@ def test_batched_expired_wait_is_reported(ctx):
     assert np.array_equal(api.lut_linear(t, None, x, None, 4, ctx=ctx), want)
 
 
+def test_batched_limit_does_not_count_the_kernels_before(ctx):
+    """A launch that waits a long time (and gives up), and behind it one with a limit a fraction of that: the second
+    is let in early, but its waits begin when the first has ended, so its result is there."""
+    L = _lib.lib()
+    rng = np.random.default_rng(6)
+    t = synth.int4_tensor(rng, 256, 256)
+    x = np.stack([synth.activations(rng, 256) for _ in range(4)])
+    w, dx, dy, dy2 = ctx.upload(t), ctx.to_device(x), ctx.malloc(4 * 256 * 4), ctx.malloc(4 * 256 * 4)
+    ctx.linear(w, dx, dy2, batch=4)
+    want = dy2.download(np.float32)
+    dy2.zero()
+    try:
+        _lib.check(L.lmb_debug_batched_waits(ctx.h, 1, 100000))
+        ctx.linear(w, dx, dy, batch=4)
+        _lib.check(L.lmb_debug_batched_waits(ctx.h, 0, 2000))
+        ctx.linear(w, dx, dy2, batch=4)
+        with pytest.raises(_lib.LutmacError) as e:
+            ctx.sync()  # the first launch's
+        assert e.value.status == _lib.ERR_TIMEOUT
+    finally:
+        _lib.check(L.lmb_debug_batched_waits(ctx.h, 0, 0))
+    assert np.array_equal(dy2.download(np.float32), want)
+    w.free()
+
+
 @pytest.mark.parametrize("head_dim,n_heads,n_kv", [(64, 8, 2), (64, 6, 1), (128, 4, 2)])
 def test_batched_attention_positions(ctx, oracle, head_dim, n_heads, n_kv):
     """The streaming attention form: chunk edges (32 and 64 positions), sequences at different positions, an empty

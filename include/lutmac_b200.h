@@ -228,6 +228,9 @@ int lmb_debug_force_plan(int R, int n_ks, int cr);
 /* Tests: from now on the batched projections' operand barriers expect `extra_arrivals` arrivals too many
  * and their waits give up after `spin_limit` polls (0: the default); 0, 0: off. */
 int lmb_debug_batched_waits(lmb_ctx *ctx, int extra_arrivals, unsigned spin_limit);
+/* Tests: from now on the batched projections take this many sequences per pass (a multiple of 4 up to 32) and
+ * this many CTAs per pass (no more than there are units of work); 0: the planner's choice. */
+int lmb_debug_batched_plan(lmb_ctx *ctx, int seqs_per_pass, int ctas);
 /* Tests: from now on the attention launches of several sequences cut the cache into `n_splits` parts, the
  * barriers that hand a ring stage back expect `extra_arrivals` arrivals too many, and waits give up after
  * `spin_limit` polls (0: the defaults).  Steps captured into graphs earlier keep what they were captured with. */

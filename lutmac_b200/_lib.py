@@ -87,6 +87,7 @@ SIGNATURES = {
     "lmb_debug_launch_timeline": (C.c_int, [vp, sz, vp, C.POINTER(sz)]),
     "lmb_debug_force_plan": (C.c_int, [C.c_int, C.c_int, C.c_int]),
     "lmb_debug_batched_waits": (C.c_int, [vp, C.c_int, C.c_uint]),
+    "lmb_debug_batched_plan": (C.c_int, [vp, C.c_int, C.c_int]),
     "lmb_debug_attn_stream": (C.c_int, [vp, C.c_int, C.c_int, C.c_uint]),
     "lmb_debug_bounds": (C.c_int, [vp, C.POINTER(C.c_ulonglong)]),
     "lmb_debug_bounds_shrink": (C.c_int, [sz]),

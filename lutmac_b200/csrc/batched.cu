@@ -405,11 +405,14 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
         before = __shfl_sync(0xffffffffu, before, 0);
         if (before != unsigned(parts - 1)) return;
         __syncwarp();
+        // Parts are added in pairs, fours and sixteens: few rows over a long K are cut into dozens of parts, and one
+        // serial fp32 chain over them had up to 1.5 times the error of the short slices of a single sequence.
 #pragma unroll
         for (int q0 = 0; q0 < NSMAX; q0 += 8) {
           if (q0 < nb) {
+            float some[8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[q0 + q] = 0.0f;
+            for (int q = 0; q < 8; ++q) v[q0 + q] = some[q] = 0.0f;
             for (int k0 = 0; k0 < parts; k0 += 4) {  // 32 loads in flight per lane
               float t[4][8];
 #pragma unroll
@@ -418,10 +421,17 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
                 for (int q = 0; q < 8; ++q)
                   t[k][q] = (k0 + k < parts && q0 + q < nb) ? __ldcg(part(k0 + k) + size_t(q0 + q) * ROWS) : 0.0f;
 #pragma unroll
-              for (int k = 0; k < 4; ++k)
+              for (int q = 0; q < 8; ++q) some[q] += (t[0][q] + t[1][q]) + (t[2][q] + t[3][q]);
+              if ((k0 & 12) == 12) {
 #pragma unroll
-                for (int q = 0; q < 8; ++q) v[q0 + q] += t[k][q];
+                for (int q = 0; q < 8; ++q) {
+                  v[q0 + q] += some[q];
+                  some[q] = 0.0f;
+                }
+              }
             }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q0 + q] += some[q];
           }
         }
       }
@@ -608,10 +618,12 @@ struct BtPlan {
 // Shared memory of one SM (228 KiB) less what the driver and the static part take.
 constexpr size_t BT_SMEM = 220 * 1024;
 
-BtPlan plan_batched(int kind, const size_t *row_tiles, int njobs, size_t bpr, size_t batch, int sm_count) {
+// force_seqs, force_ctas: sequences per pass and CTAs per pass of the test hook (0: free choice).
+BtPlan plan_batched(int kind, const size_t *row_tiles, int njobs, size_t bpr, size_t batch, int sm_count, int force_seqs, int force_ctas) {
   BtPlan pl{};
   const int W = 4 * bt_halves(kind);
-  pl.passes = int((batch + BT_MAX_SEQS - 1) / BT_MAX_SEQS);
+  const size_t most = force_seqs ? size_t(force_seqs) : size_t(BT_MAX_SEQS);
+  pl.passes = int((batch + most - 1) / most);
   const size_t per = (batch + pl.passes - 1) / pl.passes;
   pl.ns = int((per + 3) / 4 * 4);
   pl.nsmax = pl.ns <= 8 ? 8 : pl.ns <= 16 ? 16 : 32;
@@ -628,6 +640,7 @@ BtPlan plan_batched(int kind, const size_t *row_tiles, int njobs, size_t bpr, si
     return e ? size_t(std::atoi(e)) : size_t(2);
   }();
   pl.ctas = int(std::max<size_t>(1, std::min(slots / size_t(pl.passes), total / min_units)));  // per pass
+  if (force_ctas) pl.ctas = int(std::min(total, size_t(force_ctas)));
   pl.scratch = pl.ctas > 1 ? size_t(pl.passes) * pl.ctas * 2 * pl.ns * W * TILE_ROWS : 0;
   pl.counters = size_t(pl.passes) * pl.n_rg * W;
   pl.img_records = size_t(pl.passes) * pl.ns * bpr;
@@ -695,7 +708,7 @@ int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate,
   const int kind = args[0].w->kind, W = 4 * bt_halves(kind);
   size_t row_tiles[BT_MAX_JOBS];
   for (int j = 0; j < njobs; ++j) row_tiles[j] = args[j].w->row_tiles;
-  const BtPlan pl = plan_batched(kind, row_tiles, njobs, args[0].w->bpr, args[0].batch, ctx->sm_count);
+  const BtPlan pl = plan_batched(kind, row_tiles, njobs, args[0].w->bpr, args[0].batch, ctx->sm_count, ctx->batched_force_seqs, ctx->batched_force_ctas);
   if (pl.n_stages < 2) return LMB_ERR_LIMIT;
   if (pl.scratch > ctx->scratch_floats || pl.counters > ctx->n_counters || pl.img_records > ctx->xprep_blocks) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -767,6 +780,14 @@ int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate,
 }
 
 }  // namespace lmb
+
+extern "C" int lmb_debug_batched_plan(lmb_ctx *ctx, int seqs_per_pass, int ctas) {
+  LMB_REQUIRE(ctx && seqs_per_pass >= 0 && seqs_per_pass <= lmb::BT_MAX_SEQS && seqs_per_pass % 4 == 0 && ctas >= 0,
+              "lmb_debug_batched_plan: bad argument");
+  ctx->batched_force_seqs = seqs_per_pass;
+  ctx->batched_force_ctas = ctas;
+  return LMB_OK;
+}
 
 extern "C" int lmb_debug_batched_waits(lmb_ctx *ctx, int extra_arrivals, unsigned spin_limit) {
   LMB_REQUIRE(ctx && extra_arrivals >= 0, "lmb_debug_batched_waits: bad argument");

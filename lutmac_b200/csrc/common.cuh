@@ -194,6 +194,7 @@ struct lmb_ctx {
   unsigned *d_fault = nullptr;
   unsigned batched_spin_limit = 1u << 22;  // polls before a wait of the batched kernel gives up (seconds)
   int batched_extra_arrivals = 0;          // test hook, lmb_debug_batched_waits
+  int batched_force_seqs = 0, batched_force_ctas = 0;  // test hook, lmb_debug_batched_plan
   volatile unsigned *fault = nullptr;  // the flag as the host sees it
   uint64_t fault_gen = 0;              // faults reported so far: models clear their own arrival counters when it has moved
   // test hook, lmb_debug_attn_stream

@@ -36,6 +36,33 @@ def test_batched_linear_vs_fp64(ctx, oracle, kind):
         w.free()
 
 
+@pytest.mark.parametrize("M", (64, 128, 512))
+@pytest.mark.parametrize("kind", (TERNARY, INT4, INT8))
+def test_batched_error_of_few_rows_and_a_long_row(ctx, oracle, kind, M):
+    """112 blocks per row, cut over as many CTAs as there are: the fp32 error against 64 bits is that of the same
+    sequences one at a time, whose sums are short slices (both are sums of M x 8 independent errors: their norms
+    agree within a few percent when the orders are equally good, and a serial chain of 56 parts is 1.3 to 1.5 times off)."""
+    rng = np.random.default_rng(40 + kind)
+    K, batch = 28672, 8
+    t = synth.tensor(rng, kind, M, K)
+    x = np.stack([synth.activations(rng, K) for _ in range(batch)])
+    w, dx, dy = ctx.upload(t), ctx.to_device(x), ctx.malloc(batch * M * 4)
+    one = np.empty((batch, M), np.float32)
+    for q in range(batch):
+        dq = ctx.to_device(x[q])
+        ctx.linear(w, dq, dy, flags=0)
+        one[q] = dy.download(np.float32, M)
+    _lib.check(_lib.lib().lmb_debug_batched_plan(ctx.h, 8, 10000))
+    try:
+        ctx.linear(w, dx, dy, batch=batch, flags=0)
+    finally:
+        _lib.check(_lib.lib().lmb_debug_batched_plan(ctx.h, 0, 0))
+    y = dy.download(np.float32).reshape(batch, M)
+    want = np.stack([oracle.gemv_f64(kind, t.blocks, x[q], M, K) for q in range(batch)])
+    assert np.linalg.norm(y - want) < 1.15 * np.linalg.norm(one - want)
+    w.free()
+
+
 def test_batched_sums_are_deterministic_and_match_single_sequences(ctx):
     """A row group cut over many CTAs gives the same bits every time, and a sequence's result does not
     depend on what the other sequences hold (infinities and NaN among them)."""

@@ -405,14 +405,13 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
         before = __shfl_sync(0xffffffffu, before, 0);
         if (before != unsigned(parts - 1)) return;
         __syncwarp();
-        // Parts are added in pairs, fours and sixteens: few rows over a long K are cut into dozens of parts, and one
-        // serial fp32 chain over them had up to 1.5 times the error of the short slices of a single sequence.
+        // Parts are added in pairs and fours, which shortens the serial fp32 chain over them: with one addition per
+        // part, few rows over a long K (dozens of parts) had up to 1.5 times the error of a single sequence's short slices.
 #pragma unroll
         for (int q0 = 0; q0 < NSMAX; q0 += 8) {
           if (q0 < nb) {
-            float some[8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[q0 + q] = some[q] = 0.0f;
+            for (int q = 0; q < 8; ++q) v[q0 + q] = 0.0f;
             for (int k0 = 0; k0 < parts; k0 += 4) {  // 32 loads in flight per lane
               float t[4][8];
 #pragma unroll
@@ -421,17 +420,8 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
                 for (int q = 0; q < 8; ++q)
                   t[k][q] = (k0 + k < parts && q0 + q < nb) ? __ldcg(part(k0 + k) + size_t(q0 + q) * ROWS) : 0.0f;
 #pragma unroll
-              for (int q = 0; q < 8; ++q) some[q] += (t[0][q] + t[1][q]) + (t[2][q] + t[3][q]);
-              if ((k0 & 12) == 12) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                  v[q0 + q] += some[q];
-                  some[q] = 0.0f;
-                }
-              }
+              for (int q = 0; q < 8; ++q) v[q0 + q] += (t[0][q] + t[1][q]) + (t[2][q] + t[3][q]);
             }
-#pragma unroll
-            for (int q = 0; q < 8; ++q) v[q0 + q] += some[q];
           }
         }
       }

@@ -171,6 +171,7 @@ static int linear_impl(lmb_ctx *ctx, const lmb_weight *w, const float *d_bias, c
   // (lut_gemm_scalar.cpp:92-93): ternary, binary and 2-bit tensors.
   const bool auto_rot = (w->ref_kind == LMB_TERNARY || w->ref_kind == LMB_BINARY || w->ref_kind == LMB_INT2);
   a.rotate = (flags & LMB_ROTATE) || ((flags & LMB_AUTO_ROTATE) && auto_rot);
+  a.alone = true;
   return launch_gemv(ctx, &a, 1, a.rotate);
 }
 

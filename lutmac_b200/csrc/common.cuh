@@ -267,6 +267,7 @@ struct LinearArgs {
   const uint32_t *prep_in = nullptr;
   const float *prep_sumsq_in = nullptr;
   int prep_sumsq_n = 0;
+  bool alone = false;  // a call of its own, not a launch of a decode step (which form of the kernel runs: see k_gemv)
 };
 constexpr int PREP_RECORD_WORDS = 256 + 4;  // one prepared 256-block: digits, block scale, two digit-pair sums, pad
 // How the GEMV prologue forms its activations from x.

@@ -108,9 +108,16 @@ struct GemvParams {
 
 // CLUSTERED: the instantiation launched with thread-block clusters (GemvParams::cl_size); kept apart so
 // that the ordinary kernel carries none of its code.
-template <int KIND, int NSEQ, bool CLUSTERED = false>
+// ALONE: the instantiation without the normalisation, for prepared groups and single projections of one sequence.  At
+// its bound of 128 registers the kernel's main loop pays for a norm weight that is live across the wait and for the
+// scaling behind the reduction (2-bit 28672 x 8192: 26.0 -> 24.5 us without them; 5 layers of a 1.5B shape in 2 bits
+// as a group: 41.7 -> 32.6 us).
+// The launches of a decode step take the general form all the same: alternating between two kernels costs about a
+// microsecond each time (8 layers of a 1B shape: 274 us a step, 290 us with o_proj as another instantiation).
+template <int KIND, int NSEQ, bool CLUSTERED = false, bool ALONE = false>
 __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __grid_constant__ GemvParams p) {
   static_assert(!CLUSTERED || (NSEQ == 1 && kind_is_mma(KIND)), "clusters: batch 1, integer-MMA kinds");
+  static_assert(!ALONE || (NSEQ == 1 && !CLUSTERED), "the form without normalisation: one sequence, no clusters");
   // NSEQ sequences share one pass over the weights (integer-MMA kinds only: two sequences per
   // MMA); the other kinds run one sequence per CTA, blockIdx.y selecting it.
   static_assert(NSEQ == 1 || kind_is_mma(KIND), "several sequences per pass need an integer-MMA kind");
@@ -171,7 +178,7 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
 
   // so is the norm weight of the first block this warp converts
   float w8[8];
-  if (NSEQ == 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered && warp < ns) load_x8(job.x2, job.x_len, size_t(b0 + warp), lane, w8);
+  if (!ALONE && NSEQ == 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered && warp < ns) load_x8(job.x2, job.x_len, size_t(b0 + warp), lane, w8);
 
   pdl_wait();
   if (threadIdx.x == 0) {
@@ -187,7 +194,7 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
   // x * w and the row sums are multiplied by 1 / rms at the end: the sum of squares and the conversion read x
   // side by side, instead of one round trip and two barriers after the other (1B-shaped step with the
   // page-locked logits: 611 -> 558 us).
-  const bool late_rms = NSEQ == 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered;
+  const bool late_rms = !ALONE && NSEQ == 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered;
   if (NSEQ > 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered) {
     // RMSNorm of the whole input vectors, recomputed by every CTA
     float ss[NSEQ];
@@ -320,7 +327,7 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
     float v[8], nv[8];
     const int items = ns * nb;
     auto second = [&](int q, int bl) {  // norm weight, or the vector multiplied in
-      if (p.xmode == XMODE_RMSNORM) load_x8(job.x2, job.x_len, size_t(b0 + bl), lane, w8);
+      if (!ALONE && p.xmode == XMODE_RMSNORM) load_x8(job.x2, job.x_len, size_t(b0 + bl), lane, w8);
       if (p.xmode == XMODE_SILU_MUL || p.xmode == XMODE_GELU_MUL) load_x8(job.x2 + size_t(batch0 + q) * job.x_stride, job.x_len, size_t(b0 + bl), lane, w8);
     };
     if (warp < items) load_x8(x + size_t(NSEQ == 1 ? 0 : warp / ns) * job.x_stride, job.x_len, size_t(b0 + (NSEQ == 1 ? warp : warp % ns)), lane, nv);
@@ -341,7 +348,7 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
         const int nq = NSEQ == 1 ? 0 : (it + WARPS) / ns;
         load_x8(x + size_t(nq) * job.x_stride, job.x_len, size_t(b0 + (it + WARPS) - nq * ns), lane, nv);
       }
-      if (p.xmode == XMODE_RMSNORM) {
+      if (!ALONE && p.xmode == XMODE_RMSNORM) {
         const float ir = late_rms ? 1.0f : inv_rms[q];
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = v[e] * ir * w8[e];
@@ -942,7 +949,11 @@ int prepare_jobs(lmb_ctx *ctx, int kind, const LinearArgs *args, int njobs, Job 
   return LMB_OK;
 }
 
-template <int KIND, int NSEQ> int launch_params(lmb_ctx *ctx, GemvParams &p, int ctas, int s_max, size_t batch) {
+// Binary has no form without the normalisation: there it measured slower (28672 x 8192: 18.7 us against 16.3).
+constexpr bool has_alone_form(int kind) { return kind != DK_BINARY_MMA; }
+
+// alone: not part of a decode step.
+template <int KIND, int NSEQ> int launch_params(lmb_ctx *ctx, GemvParams &p, int ctas, int s_max, size_t batch, bool alone) {
   p.batch = int(batch);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(ctas), unsigned((batch + NSEQ - 1) / NSEQ));
@@ -975,39 +986,46 @@ template <int KIND, int NSEQ> int launch_params(lmb_ctx *ctx, GemvParams &p, int
       return LMB_OK;
     }
   }
+  if constexpr (NSEQ == 1 && has_alone_form(KIND)) {
+    if (alone && p.xmode == XMODE_PLAIN) {
+      LMB_CUDA(cudaLaunchKernelEx(&cfg, k_gemv<KIND, 1, false, true>, p));
+      ctx->launches++;
+      return LMB_OK;
+    }
+  }
   LMB_CUDA(cudaLaunchKernelEx(&cfg, k_gemv<KIND, NSEQ>, p));
   ctx->launches++;
   return LMB_OK;
 }
 
-template <int KIND> int launch_params_mma(lmb_ctx *ctx, GemvParams &p, int ctas, int s_max, size_t batch) {
+template <int KIND> int launch_params_mma(lmb_ctx *ctx, GemvParams &p, int ctas, int s_max, size_t batch, bool alone) {
   switch (seqs_per_pass(KIND, batch)) {
-  case 1: return launch_params<KIND, 1>(ctx, p, ctas, s_max, batch);
-  case 2: return launch_params<KIND, 2>(ctx, p, ctas, s_max, batch);
+  case 1: return launch_params<KIND, 1>(ctx, p, ctas, s_max, batch, alone);
+  case 2: return launch_params<KIND, 2>(ctx, p, ctas, s_max, batch, alone);
   case 4:
-    if constexpr (max_seqs_per_pass(KIND) >= 4) return launch_params<KIND, 4>(ctx, p, ctas, s_max, batch);
+    if constexpr (max_seqs_per_pass(KIND) >= 4) return launch_params<KIND, 4>(ctx, p, ctas, s_max, batch, alone);
     return LMB_ERR_STATE;
   default:
-    if constexpr (max_seqs_per_pass(KIND) >= 8) return launch_params<KIND, 8>(ctx, p, ctas, s_max, batch);
+    if constexpr (max_seqs_per_pass(KIND) >= 8) return launch_params<KIND, 8>(ctx, p, ctas, s_max, batch, alone);
     return LMB_ERR_STATE;
   }
 }
 
-int launch_params_kind(lmb_ctx *ctx, int kind, GemvParams &p, int ctas, int s_max, size_t batch) {
+int launch_params_kind(lmb_ctx *ctx, int kind, GemvParams &p, int ctas, int s_max, size_t batch, bool alone) {
   switch (kind) {
-  case LMB_TERNARY: return launch_params<LMB_TERNARY, 1>(ctx, p, ctas, s_max, batch);
-  case LMB_BINARY: return launch_params<LMB_BINARY, 1>(ctx, p, ctas, s_max, batch);
-  case LMB_INT2: return launch_params<LMB_INT2, 1>(ctx, p, ctas, s_max, batch);
-  case LMB_INT3: return launch_params<LMB_INT3, 1>(ctx, p, ctas, s_max, batch);
-  case LMB_INT8: return launch_params<LMB_INT8, 1>(ctx, p, ctas, s_max, batch);
-  case LMB_INT4: return launch_params_mma<LMB_INT4>(ctx, p, ctas, s_max, batch);
-  case DK_TERNARY_MMA: return launch_params_mma<DK_TERNARY_MMA>(ctx, p, ctas, s_max, batch);
-  case DK_INT2_MMA: return launch_params_mma<DK_INT2_MMA>(ctx, p, ctas, s_max, batch);
-  case DK_BINARY_MMA: return launch_params_mma<DK_BINARY_MMA>(ctx, p, ctas, s_max, batch);
-  case LMB_INT5: return launch_params_mma<LMB_INT5>(ctx, p, ctas, s_max, batch);
-  case LMB_INT6: return launch_params_mma<LMB_INT6>(ctx, p, ctas, s_max, batch);
-  case DK_INT8_MMA: return launch_params_mma<DK_INT8_MMA>(ctx, p, ctas, s_max, batch);
-  case DK_INT3_MMA: return launch_params_mma<DK_INT3_MMA>(ctx, p, ctas, s_max, batch);
+  case LMB_TERNARY: return launch_params<LMB_TERNARY, 1>(ctx, p, ctas, s_max, batch, alone);
+  case LMB_BINARY: return launch_params<LMB_BINARY, 1>(ctx, p, ctas, s_max, batch, alone);
+  case LMB_INT2: return launch_params<LMB_INT2, 1>(ctx, p, ctas, s_max, batch, alone);
+  case LMB_INT3: return launch_params<LMB_INT3, 1>(ctx, p, ctas, s_max, batch, alone);
+  case LMB_INT8: return launch_params<LMB_INT8, 1>(ctx, p, ctas, s_max, batch, alone);
+  case LMB_INT4: return launch_params_mma<LMB_INT4>(ctx, p, ctas, s_max, batch, alone);
+  case DK_TERNARY_MMA: return launch_params_mma<DK_TERNARY_MMA>(ctx, p, ctas, s_max, batch, alone);
+  case DK_INT2_MMA: return launch_params_mma<DK_INT2_MMA>(ctx, p, ctas, s_max, batch, alone);
+  case DK_BINARY_MMA: return launch_params_mma<DK_BINARY_MMA>(ctx, p, ctas, s_max, batch, alone);
+  case LMB_INT5: return launch_params_mma<LMB_INT5>(ctx, p, ctas, s_max, batch, alone);
+  case LMB_INT6: return launch_params_mma<LMB_INT6>(ctx, p, ctas, s_max, batch, alone);
+  case DK_INT8_MMA: return launch_params_mma<DK_INT8_MMA>(ctx, p, ctas, s_max, batch, alone);
+  case DK_INT3_MMA: return launch_params_mma<DK_INT3_MMA>(ctx, p, ctas, s_max, batch, alone);
   default: set_last_error("launch_gemv: kind has no device kernel"); return LMB_ERR_ARG;
   }
 }
@@ -1018,6 +1036,8 @@ template <int KIND> int configure_mma() {
   const int small = 64 * 1024, large = 100 * 1024;
   LMB_CUDA(cudaFuncSetAttribute(k_gemv<KIND, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, small));
   LMB_CUDA(cudaFuncSetAttribute(k_gemv<KIND, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, small));
+  if constexpr (has_alone_form(KIND))
+    LMB_CUDA(cudaFuncSetAttribute(k_gemv<KIND, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, small));
   LMB_CUDA(cudaFuncSetAttribute(k_gemv<KIND, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, small));
   if constexpr (max_seqs_per_pass(KIND) >= 4)
     LMB_CUDA(cudaFuncSetAttribute(k_gemv<KIND, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, large));
@@ -1030,10 +1050,15 @@ int configure_gemv(lmb_ctx *ctx) {
   (void)ctx;
   const int bytes = 64 * 1024;
   LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_TERNARY, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_TERNARY, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_BINARY, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_BINARY, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_INT2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_INT2, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_INT3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_INT3, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_INT8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  LMB_CUDA(cudaFuncSetAttribute(k_gemv<LMB_INT8, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   int st = configure_mma<LMB_INT4>();
   if (st == LMB_OK) st = configure_mma<DK_TERNARY_MMA>();
   if (st == LMB_OK) st = configure_mma<DK_INT2_MMA>();
@@ -1122,7 +1147,7 @@ int launch_gemv(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, in
     p.prep = args[0].prep_in;
     p.prep_sumsq = args[0].prep_sumsq_in;
     p.prep_sumsq_n = args[0].prep_sumsq_n;
-    return launch_params_kind(ctx, kind, p, ctas, s_max, 1);
+    return launch_params_kind(ctx, kind, p, ctas, s_max, 1, false);
   }
   // Batches of three or more sequences whose jobs read one input: convert the activations once
   // for the whole launch instead of once per CTA.
@@ -1151,7 +1176,7 @@ int launch_gemv(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, in
       p.prep = ctx->xprep;
     }
   }
-  return launch_params_kind(ctx, kind, p, ctas, s_max, args[0].batch);
+  return launch_params_kind(ctx, kind, p, ctas, s_max, args[0].batch, args[0].alone);
 }
 
 }  // namespace lmb
@@ -1250,7 +1275,7 @@ int lmb_group_launch(lmb_ctx *ctx, lmb_group *g) {
   p.prep_sumsq = nullptr;
   p.prep_sumsq_n = 0;
   p.cl_size = 0;
-  return launch_params_kind(ctx, g->kind, p, g->ctas, g->s_max, 1);
+  return launch_params_kind(ctx, g->kind, p, g->ctas, g->s_max, 1, true);
 }
 
 int lmb_group_destroy(lmb_group *g) {
@@ -1475,7 +1500,7 @@ int lmb_linear_static_scratch(const lmb_weight *w, const float *d_bias, const fl
   launch_ctx.device = dev;
   launch_ctx.stream = stream;
   launch_ctx.pdl = false;
-  return launch_params_kind(&launch_ctx, kind, p, pl.ctas, pl.S, 1);
+  return launch_params_kind(&launch_ctx, kind, p, pl.ctas, pl.S, 1, true);
 }
 
 }  // extern "C"

@@ -750,6 +750,13 @@ inline bool clusters_allowed() {
 // Resident CTAs per SM of k_gemv<kind> (register limited), used to count waves.
 int ctas_per_sm(int kind) { return kind_info(kind).lut ? 3 : 2; }
 
+// Time of a CTA of S blocks whose row-tiles are shared by `wpr` warps each, in units of "one warp evaluates one
+// 256-column block": the main loop, the conversion of the activations, a fixed part and the hand-off of a K split.
+double cta_units(size_t S, size_t wpr, size_t n_ks, int nseq, size_t cr) {
+  const size_t converted = cr ? (S + cr - 1) / cr : S;  // blocks this CTA converts itself
+  return double((S + wpr - 1) / wpr) + 1.5 * nseq * double((converted + 7) / 8) + 1.5 + (cr ? 3.0 : 0.0) + (n_ks > 1 ? (cr ? 0.8 : 2.5) : 0.0);
+}
+
 // Chooses R (row-tiles per CTA: 8, 4, 2 or 1; the 8 warps of a CTA then share a row-tile
 // 1, 2, 4 or 8 ways along K, which costs only a shared-memory reduction), the K split over CTAs
 // and whether the CTAs form thread-block clusters (K slices added up through distributed shared
@@ -767,7 +774,6 @@ Plan make_plan(int kind, size_t row_tiles, size_t bpr, size_t batch, int sm_coun
   // 48 KiB of tables / activations per CTA (96 KiB when 4 or 8 sequences share a pass)
   const size_t s_cap = lut ? 12 : nseq == 1 ? 48 : nseq == 8 ? 12 : 24;
   const size_t slots = size_t(sm_count) * (min_ctas(kind, nseq) == 1 ? 1 : ctas_per_sm(kind));
-  const double prologue_per_block = 1.5 * nseq, fixed = 1.5, split_cost = 2.5, cluster_sync = 3.0, cluster_split = 0.8;
   const bool throughput = (other_row_tiles + 7) / 8 * batch >= 2 * slots;
   const bool may_cluster = cluster != 0 && kind_is_mma(kind) && nseq == 1 && batch == 1 && bpr <= size_t(MAX_CLUSTER_BLOCKS) &&
                            (clusters_allowed() || (force.on && force.cr > 0));
@@ -804,10 +810,7 @@ Plan make_plan(int kind, size_t row_tiles, size_t bpr, size_t batch, int sm_coun
         const size_t own = n_rgp * n_ks * batch;
         // other jobs of the launch are assumed to be cut the same way
         const size_t other_ctas = (other_row_tiles + R - 1) / R * n_ks * batch;
-        const double per_warp = double((S + wpr - 1) / wpr);
-        const size_t converted = cr ? (S + size_t(cr) - 1) / size_t(cr) : S;  // blocks this CTA converts itself
-        const double cta_time = per_warp + prologue_per_block * double((converted + 7) / 8) + fixed + (cr ? cluster_sync : 0.0) +
-                                (n_ks > 1 ? (cr ? cluster_split : split_cost) : 0.0);
+        const double cta_time = cta_units(S, wpr, n_ks, nseq, size_t(cr));
         // with plenty of work from other jobs (even cut 8 row-tiles per CTA) the GPU is busy anyway:
         // minimise this job's total CTA time; otherwise minimise the time until its last CTA finishes
         const double cost = (throughput ? double(own) * cta_time / double(slots)
@@ -826,6 +829,80 @@ Plan make_plan(int kind, size_t row_tiles, size_t bpr, size_t batch, int sm_coun
     }
   }
   return best;
+}
+
+// Prepared groups: make_plan plans a job as if the others were cut like it, so a K split of one job with few rows and a
+// long K (down_proj) looks like a second wave of the whole group, and the launch lasts as long as that job's chain:
+// 3 layers of a 1.5B shape in 2 bits took as long as 7 (33 to 44 us, depending on where the long CTAs land),
+// 4 layers 20.  Where the longest CTA is well above the average load of a slot, the group is planned as a whole
+// instead: every job takes its cheapest split whose CTAs are no longer than a bound, for the bound that makes
+// max(bound, total work / slots) smallest.  In us: 1.5B shape, 2 bits, 3 / 5 / 8 layers 44.4 / 32.6 / 34.8 -> 18.8 / 23.3 /
+// 32.5; 1B shape, 4 bits, 1 / 3 / 6 layers 12.7 / 30.3 / 34.8 -> 8.6 / 23.0 / 32.4; no group of 1 to 8 layers of either shape slower.
+void balance_group(int kind, const LinearArgs *args, std::vector<Plan> &plans, int sm_count) {
+  const size_t n = plans.size();
+  const double slots = double(size_t(sm_count) * (min_ctas(kind, 1) == 1 ? 1 : ctas_per_sm(kind)));
+  const size_t s_cap = kind_info(kind).lut ? 12 : 48;
+  double longest = 0.0, work = 0.0;
+  for (const Plan &pl : plans) {
+    const double t = cta_units(size_t(pl.S), size_t(8 / pl.R), size_t(pl.n_ks), 1, 0);
+    longest = std::max(longest, t);
+    work += t * pl.ctas;
+  }
+  if (g_plan_force.on || longest <= 1.5 * work / slots) return;
+  struct Shape {
+    size_t row_tiles, bpr, count;
+    std::vector<std::pair<double, Plan>> cuts;  // CTA time, plan
+    Plan best;
+  };
+  std::vector<Shape> shapes;
+  std::vector<size_t> of(n);
+  std::vector<double> bounds;
+  for (size_t j = 0; j < n; ++j) {
+    const lmb_weight *w = args[j].w;
+    size_t k = 0;
+    while (k < shapes.size() && (shapes[k].row_tiles != w->row_tiles || shapes[k].bpr != w->bpr)) ++k;
+    of[j] = k;
+    if (k < shapes.size()) {
+      ++shapes[k].count;
+      continue;
+    }
+    shapes.push_back({w->row_tiles, w->bpr, 1, {}, {}});
+    for (int R = 8; R >= 1; R >>= 1) {
+      if (size_t(R) > w->row_tiles && R > 1) continue;
+      for (size_t n_ks = 1; n_ks <= w->bpr; ++n_ks) {
+        const size_t S = (w->bpr + n_ks - 1) / n_ks;
+        if (S > s_cap || (w->bpr + S - 1) / S != n_ks) continue;
+        const size_t n_rg = (w->row_tiles + size_t(R) - 1) / size_t(R);
+        const double t = cta_units(S, size_t(8 / R), n_ks, 1, 0);
+        shapes[k].cuts.push_back({t, Plan{R, int(S), int(n_rg), int(n_ks), int(n_rg * n_ks), 0}});
+        bounds.push_back(t);
+      }
+    }
+  }
+  double best = std::max(longest, work / slots);
+  bool found = false;
+  std::vector<Plan> pick(shapes.size());
+  for (double bound : bounds) {
+    double total = 0.0;
+    bool ok = true;
+    for (size_t k = 0; k < shapes.size() && ok; ++k) {
+      double least = 1e30;
+      for (const auto &c : shapes[k].cuts)
+        if (c.first <= bound && c.first * c.second.ctas < least) {
+          least = c.first * c.second.ctas;
+          pick[k] = c.second;
+        }
+      ok = least < 1e30;
+      total += least * double(shapes[k].count);
+    }
+    if (ok && std::max(bound, total / slots) < best) {
+      best = std::max(bound, total / slots);
+      found = true;
+      for (size_t k = 0; k < shapes.size(); ++k) shapes[k].best = pick[k];
+    }
+  }
+  if (found)
+    for (size_t j = 0; j < n; ++j) plans[j] = shapes[of[j]].best;
 }
 
 // Sequences that share one pass over the weights (template parameter NSEQ of k_gemv).
@@ -866,6 +943,10 @@ int prepare_jobs(lmb_ctx *ctx, int kind, const LinearArgs *args, int njobs, Job 
     const lmb_weight *w = args[j].w;
     const size_t others = total_rt - w->row_tiles;
     plans[size_t(j)] = make_plan(kind, w->row_tiles, w->bpr, ny, ctx->sm_count, others, nseq, args[j].next_prep != nullptr, cluster);
+  }
+  if (cta_map) balance_group(kind, args, plans, ctx->sm_count);
+  for (int j = 0; j < njobs; ++j) {
+    const lmb_weight *w = args[j].w;
     static const bool print_plans = std::getenv("LMB_PLAN_PRINT") != nullptr;  // debugging: the work split of every launch
     if (print_plans)
       std::fprintf(stderr, "lmb plan: kind %d job %d/%d rows %zu blocks/row %zu batch %zu: R %d S %d K slices %d, row groups per cluster %d, %d CTAs\n",

@@ -238,6 +238,28 @@ def test_prepared_group_equals_single_launches(ctx, oracle, kind):
             assert rel_l2(dy.download(np.float32), want) < TOL, (KIND_NAMES[kind], t.M, t.K)
 
 
+@pytest.mark.parametrize("kind", (TERNARY, INT2, INT4, INT8, BINARY))
+def test_group_with_one_long_job(ctx, oracle, kind):
+    """Many short jobs and one of few rows and 35 blocks per row, whose CTAs would outlast the launch: the group is cut
+    as a whole (other K splits than the jobs have alone), twice with the same bits, against the fp64 truth."""
+    rng = np.random.default_rng(60 + kind)
+    shapes = [(256, 1536)] * 12 + [(1500, 8960), (33, 300), (1500, 8960)]
+    ts = [synth.tensor(rng, kind, M, K) for M, K in shapes]
+    xs = [synth.activations(rng, K) for _, K in shapes]
+    ws = [ctx.upload(t) for t in ts]
+    dxs, dys = [ctx.to_device(x) for x in xs], [ctx.malloc(M * 4) for M, _ in shapes]
+    g = api.Group(ctx, ws, dxs, dys, flags=0)
+    runs = []
+    for _ in range(2):
+        g.launch()
+        runs.append([dy.download(np.float32) for dy in dys])
+    for i, (M, K) in enumerate(shapes):
+        assert np.array_equal(runs[0][i], runs[1][i]), (i, M, K)
+        x = np.zeros(blocks_per_row(K) * 256, np.float32)
+        x[:K] = xs[i]
+        assert rel_l2(runs[0][i], oracle.gemv_f64(kind, ts[i].blocks, x, M, K)) < 1e-6, (i, M, K)  # fp32 sums over 35 blocks
+
+
 def test_split_k_is_deterministic(ctx):
     rng = np.random.default_rng(11)
     t = synth.int4_tensor(rng, 64, 8192)  # few rows, many blocks: K is split over CTAs

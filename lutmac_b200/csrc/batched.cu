@@ -27,7 +27,6 @@
 // Roles: 4 * H worker warps (a 32-row tile each), one producer thread (bulk copies), one MMA thread.
 // Every wait is bounded: on expiry the kernel raises the context's fault flag and leaves in order.
 #include <algorithm>
-#include <cstdlib>
 
 #include "decode_device.cuh"
 #include "gemv_units.cuh"
@@ -603,38 +602,93 @@ struct BtPlan {
   int passes, ns, n_rg, ctas, n_stages, nsmax;
   unsigned stage_bytes;
   size_t scratch, counters, img_records;
+  float us;  // estimated time of both kernels of the launch
 };
 
 // Shared memory of one SM (228 KiB) less what the driver and the static part take.
 constexpr size_t BT_SMEM = 220 * 1024;
 
-// force_seqs, force_ctas: sequences per pass and CTAs per pass of the test hook (0: free choice).
+// Estimate of a launch in microseconds, fitted to 14,700 timed launches (64 to 28672 rows x 300 to 28672 columns,
+// 4 to 32 sequences, every split).  What a CTA takes per unit of work in the forms for 8, 16 and 32 sequences:
+constexpr float BT_PART_US[3] = {0.137f, 0.295f, 0.58f};  // reading one part of a row group back
+constexpr float BT_FORM_US[3] = {0.0f, 1.1f, 3.7f};       // fixed part beyond the smallest form's
+constexpr float BT_MERGE_US = 1.5f, BT_FLAT_US = 2.0f, BT_WAVE_US = 3.5f;
+constexpr float BT_SHARED_SM = 1.3f;  // a unit's time with a second CTA on the SM
+// two launches, operand images, first copies
+constexpr float BT_BASE_US = 4.0f, BT_BASE_INT2_US = 4.4f, BT_BASE_INT8_US = 2.7f;
+float bt_unit_us(int kind, int form) {
+  switch (kind) {
+  case DK_INT2_MMA: return form == 0 ? 2.0f : form == 1 ? 2.1f : 3.2f;    // two planes
+  case DK_INT3_MMA: return form == 0 ? 1.45f : form == 1 ? 1.5f : 1.95f;  // three bit planes put together in registers
+  case DK_INT8_MMA: return 1.3f;                                          // 128 rows of 8 KiB a tile
+  case LMB_INT5:
+  case LMB_INT6: return form == 0 ? 1.0f : 1.5f;
+  default: return form == 2 ? 1.4f : 1.07f;
+  }
+}
+
+// Sequences per pass and CTAs per pass.  More passes than the 32 sequences a pass can hold need read the weights
+// again (from L2 when the passes run side by side) but fill the GPU where rows are few and take the leaner forms.
+// A row group is cut into equal parts, as many as balance the units of a CTA against reading the parts back
+// (about sqrt(blocks x 0.14) units); or all units into as many ranges as CTAs fit (flat), where that shortens the
+// longest range by more than the second merge of a CTA that then holds the end of one row group and the start of the next.
+// Against one pass of all sequences and at least two units per CTA, in us: ternary 64 x 1536, 32 sequences 13.1 -> 7.2;
+// 512 x 28672, 32 sequences 50.4 -> 21.4; 2-bit 1536 x 8960, 32 sequences 30.8 -> 21.3; 4-bit 8192 x 1536, 16 sequences
+// 9.9 -> 9.5.  The measured best over all splits is 0.7 % less on average.
+// force_seqs, force_ctas: sequences and CTAs per pass of the test hook (0: free choice).
 BtPlan plan_batched(int kind, const size_t *row_tiles, int njobs, size_t bpr, size_t batch, int sm_count, int force_seqs, int force_ctas) {
-  BtPlan pl{};
   const int W = 4 * bt_halves(kind);
-  const size_t most = force_seqs ? size_t(force_seqs) : size_t(BT_MAX_SEQS);
-  pl.passes = int((batch + most - 1) / most);
-  const size_t per = (batch + pl.passes - 1) / pl.passes;
-  pl.ns = int((per + 3) / 4 * 4);
-  pl.nsmax = pl.ns <= 8 ? 8 : pl.ns <= 16 ? 16 : 32;
-  for (int j = 0; j < njobs; ++j) pl.n_rg += int((row_tiles[j] + W - 1) / W);
-  // the 128 bytes behind an image keep the reads of unused columns' scales inside the stage
-  pl.stage_bytes = unsigned((W * tile_bytes(kind) + 127) / 128 * 128 + (size_t(pl.ns) * BT_SEQ_BYTES + 128 + 127) / 128 * 128);
-  const size_t tmem_ctas = 512 / size_t(bt_tmem_cols(kind, pl.nsmax));
-  // two CTAs per SM where TMEM and shared memory hold two with two stages each
-  const size_t per_sm = tmem_ctas > 1 && 2 * pl.stage_bytes * 2 + 8192 <= BT_SMEM ? 2 : 1;
-  pl.n_stages = int(std::min<size_t>(BT_MAX_STAGES, (BT_SMEM / per_sm - 2048) / pl.stage_bytes));
-  const size_t total = size_t(pl.n_rg) * bpr, slots = size_t(sm_count) * per_sm;
-  static const size_t min_units = [] {
-    const char *e = std::getenv("LMB_BT_MIN_UNITS");
-    return e ? size_t(std::atoi(e)) : size_t(2);
-  }();
-  pl.ctas = int(std::max<size_t>(1, std::min(slots / size_t(pl.passes), total / min_units)));  // per pass
-  if (force_ctas) pl.ctas = int(std::min(total, size_t(force_ctas)));
-  pl.scratch = pl.ctas > 1 ? size_t(pl.passes) * pl.ctas * 2 * pl.ns * W * TILE_ROWS : 0;
-  pl.counters = size_t(pl.passes) * pl.n_rg * W;
-  pl.img_records = size_t(pl.passes) * pl.ns * bpr;
-  return pl;
+  size_t n_rg = 0;
+  for (int j = 0; j < njobs; ++j) n_rg += (row_tiles[j] + W - 1) / W;
+  const size_t total = n_rg * bpr;
+  const float base = kind == DK_INT8_MMA ? BT_BASE_INT8_US : kind == DK_INT2_MMA ? BT_BASE_INT2_US : BT_BASE_US;
+  BtPlan best{};
+  for (int form = 0; form < 3; ++form) {
+    const size_t most = force_seqs ? size_t(force_seqs) : size_t(8) << form;
+    if (force_seqs ? form > 0 : form > 0 && batch <= most / 2) break;  // the form before holds all sequences
+    BtPlan pl{};
+    pl.n_rg = int(n_rg);
+    pl.passes = int((batch + most - 1) / most);
+    const size_t per = (batch + pl.passes - 1) / pl.passes;
+    pl.ns = int((per + 3) / 4 * 4);
+    const int f = pl.ns <= 8 ? 0 : pl.ns <= 16 ? 1 : 2;
+    pl.nsmax = 8 << f;
+    // the 128 bytes behind an image keep the reads of unused columns' scales inside the stage
+    pl.stage_bytes = unsigned((W * tile_bytes(kind) + 127) / 128 * 128 + (size_t(pl.ns) * BT_SEQ_BYTES + 128 + 127) / 128 * 128);
+    const size_t tmem_ctas = 512 / size_t(bt_tmem_cols(kind, pl.nsmax));
+    // two CTAs per SM where TMEM and shared memory hold two with two stages each
+    const size_t per_sm = tmem_ctas > 1 && 2 * pl.stage_bytes * 2 + 8192 <= BT_SMEM ? 2 : 1;
+    pl.n_stages = int(std::min<size_t>(BT_MAX_STAGES, (BT_SMEM / per_sm - 2048) / pl.stage_bytes));
+    const size_t slots = size_t(sm_count) * per_sm, mine = std::max<size_t>(1, slots / size_t(pl.passes));
+    auto consider = [&](size_t ctas, size_t units, size_t parts, bool flat) {
+      const size_t all = ctas * size_t(pl.passes), waves = (all + slots - 1) / slots;
+      const float unit = bt_unit_us(kind, f) * (all > size_t(sm_count) ? BT_SHARED_SM : 1.0f);
+      const float us = base + 0.015f * float(batch) + BT_FORM_US[f] + float(waves * units) * unit +
+                       (parts > 1 ? BT_MERGE_US + BT_PART_US[f] * float(parts) : 0.0f) + (flat ? BT_FLAT_US : 0.0f) +
+                       BT_WAVE_US * float(waves - 1);
+      if (best.ctas == 0 || us < best.us) {
+        best = pl;
+        best.ctas = int(ctas);
+        best.us = us;
+      }
+    };
+    if (force_ctas) {
+      consider(std::min(total, size_t(force_ctas)), 1, 1, false);
+      continue;
+    }
+    for (size_t parts = 1; parts <= bpr && n_rg * parts <= mine;) {
+      const size_t units = (bpr + parts - 1) / parts;
+      consider(n_rg * parts, units, parts, false);
+      if (units == 1) break;
+      parts = (bpr + units - 2) / (units - 1);  // the next shorter longest part
+    }
+    const size_t ctas = std::min(mine, total), units = (total + ctas - 1) / ctas;
+    if (ctas % n_rg != 0) consider(ctas, units, std::min(bpr, (bpr + total / ctas - 1) / (total / ctas) + 1), true);
+  }
+  best.scratch = best.ctas > 1 ? size_t(best.passes) * best.ctas * 2 * best.ns * W * TILE_ROWS : 0;
+  best.counters = size_t(best.passes) * best.n_rg * W;
+  best.img_records = size_t(best.passes) * best.ns * bpr;
+  return best;
 }
 
 template <int KIND, int NSMAX> int launch_one(lmb_ctx *ctx, const BtParams &p, const BtPlan &pl) {
@@ -678,14 +732,10 @@ int configure_batched() {
   return st;
 }
 
-// Whether a launch takes the batched kernel: several sequences, an integer tensor-core layout, one input for
+// Whether the batched kernel can serve a launch: several sequences, an integer tensor-core layout, one input for
 // all jobs, ordinary output.
 bool batched_possible(const LinearArgs *args, int njobs) {
-  static const size_t min_batch = [] {
-    const char *e = std::getenv("LMB_BT_MIN_BATCH");
-    return e ? size_t(std::atoi(e)) : size_t(3);
-  }();
-  if (!kind_is_mma(args[0].w->kind) || args[0].batch < min_batch || njobs > BT_MAX_JOBS) return false;
+  if (!kind_is_mma(args[0].w->kind) || args[0].batch < 3 || njobs > BT_MAX_JOBS) return false;
   for (int j = 0; j < njobs; ++j)
     if (args[j].to_peers || args[j].prep_in || args[j].next_prep || args[j].x != args[0].x || args[j].x2 != args[0].x2 ||
         args[j].x_len != args[0].x_len || args[j].x_stride != args[0].x_stride || args[j].w->bpr != args[0].w->bpr)
@@ -693,13 +743,14 @@ bool batched_possible(const LinearArgs *args, int njobs) {
   return true;
 }
 
-// LMB_ERR_LIMIT: the workspaces would have to grow while the stream is capturing; nothing was launched.
-int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, int xmode, float eps) {
+// LMB_ERR_LIMIT, and nothing launched: the estimate is above limit_us, or the workspaces would have to grow while
+// the stream is capturing.
+int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, int xmode, float eps, float limit_us) {
   const int kind = args[0].w->kind, W = 4 * bt_halves(kind);
   size_t row_tiles[BT_MAX_JOBS];
   for (int j = 0; j < njobs; ++j) row_tiles[j] = args[j].w->row_tiles;
   const BtPlan pl = plan_batched(kind, row_tiles, njobs, args[0].w->bpr, args[0].batch, ctx->sm_count, ctx->batched_force_seqs, ctx->batched_force_ctas);
-  if (pl.n_stages < 2) return LMB_ERR_LIMIT;
+  if (pl.n_stages < 2 || (pl.us > limit_us && !ctx->batched_force_seqs)) return LMB_ERR_LIMIT;
   if (pl.scratch > ctx->scratch_floats || pl.counters > ctx->n_counters || pl.img_records > ctx->xprep_blocks) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     LMB_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));

@@ -275,10 +275,10 @@ enum { XMODE_PLAIN = 0, XMODE_RMSNORM = 1, XMODE_SILU_MUL = 2, XMODE_GELU_MUL = 
 int configure_gemv(lmb_ctx *ctx);
 int launch_tp_sum_prepare(lmb_ctx *ctx, float *d_hidden, const float *d_w, bool rotate, uint32_t *prep, float *sumsq, size_t h);
 int launch_gemv(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, int xmode = XMODE_PLAIN, float eps = 0.0f);
-// Several sequences per launch on tcgen05 (batched.cu); LMB_ERR_LIMIT: not while capturing with these workspaces.
+// Several sequences per launch on tcgen05 (batched.cu); LMB_ERR_LIMIT: nothing launched, take the warp-level kernel.
 int configure_batched();
 bool batched_possible(const LinearArgs *args, int njobs);
-int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, int xmode, float eps);
+int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, int xmode, float eps, float limit_us);
 int launch_fwht256(lmb_ctx *ctx, float *d_x, size_t n);
 int launch_debug_luts(lmb_ctx *ctx, const float *d_x, size_t x_len, bool rotate, float *d_out);
 

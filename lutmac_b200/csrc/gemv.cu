@@ -31,6 +31,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -588,6 +589,7 @@ __global__ void __launch_bounds__(THREADS) k_prepare_x(const float *x, const flo
   __shared__ int aux2[WARPS][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.y;
   const float *xq = x + size_t(q) * x_stride;
+  pdl_wait();  // the input, and the launch before may still read the records
   float inv_rms = 1.0f;
   if (xmode == XMODE_RMSNORM) {
     float ss = 0.0f;
@@ -912,6 +914,49 @@ int seqs_per_pass(int kind, size_t batch) {
   return n < max_seqs_per_pass(kind) ? n : max_seqs_per_pass(kind);
 }
 
+// Estimated microseconds of a warp-level launch for several sequences, conversion of the activations included
+// (fitted to 4,900 timed launches of 3 to 32 sequences; 5 % off on average).
+float warp_level_us(int kind, const LinearArgs *args, int njobs, int sm_count) {
+  const size_t batch = args[0].batch;
+  const int nseq = seqs_per_pass(kind, batch);
+  const size_t ny = (batch + size_t(nseq) - 1) / size_t(nseq), slots = size_t(sm_count) * (min_ctas(kind, nseq) == 1 ? 1 : 2);
+  size_t total_rt = 0, ctas = 0, units = 1, blocks = 1, ks = 1;
+  for (int j = 0; j < njobs; ++j) total_rt += args[j].w->row_tiles;
+  for (int j = 0; j < njobs; ++j) {
+    const Plan pl = make_plan(kind, args[j].w->row_tiles, args[j].w->bpr, ny, sm_count, total_rt - args[j].w->row_tiles, nseq);
+    ctas += size_t(pl.n_rg) * size_t(pl.n_ks) * ny;
+    const size_t wpr = size_t(8 / pl.R);
+    units = std::max(units, (size_t(pl.S) + wpr - 1) / wpr);
+    blocks = std::max(blocks, size_t(pl.S));
+    ks = std::max(ks, size_t(pl.n_ks));
+  }
+  const float waves = float((ctas + slots - 1) / slots), split = ks > 1 ? 2.0f : 0.0f;
+  const bool two = ctas > size_t(sm_count) && slots > size_t(sm_count);  // two CTAs on an SM
+  const float many = ks > 1 ? float(ks) : 0.0f;
+  if (nseq == 2) {
+    const float unit = kind == LMB_INT5 ? 1.3f : 1.6f;
+    return 2.3f + split + 0.18f * many + 1.5f * (waves - 1.0f) + waves * (unit * float(units) + 0.12f * float(blocks)) +
+           (two ? 0.9f : 0.0f);
+  }
+  if (kind == DK_INT8_MMA) return 8.6f + 0.5f * split + 0.33f * many + 11.3f * (waves - 1.0f) + waves * (1.5f * float(units) - 0.35f * float(blocks));
+  const float unit = kind == DK_INT2_MMA ? (two ? 1.95f : 2.15f) : kind == LMB_INT4 ? (two ? 1.5f : 1.9f) : (two ? 1.1f : 1.6f);
+  const float block = kind == DK_INT2_MMA ? 0.02f : kind == LMB_INT4 ? 0.0f : 0.1f;
+  return (batch == 4 ? 4.1f : 3.1f) + 1.75f * split + 0.34f * many + waves * (unit * float(units) + block * float(blocks)) + (two ? 1.45f : 0.0f);
+}
+
+// Small launches, where a launch costs about what the estimates cost to make: the warp-level kernel keeps them.
+// 3 or 4 sequences: up to 8 blocks per row, where it needs no K split (ternary 512 x 2048, 3 sequences: 6.9 us
+// against 7.6; 28672 x 2048: 11.0 against 14.1; 512 x 4096: 9.9 against 8.7).  3-, 5- and 6-bit kinds: below
+// 2000 passes over a tile (int3 512 x 1536, 8 sequences: 4.5 us against 8.1).
+bool batched_worth_asking(int kind, const LinearArgs *args, int njobs) {
+  if (max_seqs_per_pass(kind) <= 2) {
+    size_t tiles = 0;
+    for (int j = 0; j < njobs; ++j) tiles += args[j].w->row_tiles;
+    return tiles * args[0].w->bpr * ((args[0].batch + 1) / 2) >= 2000;
+  }
+  return args[0].batch > 4 || args[0].w->bpr > 8;
+}
+
 // Plans every job of a launch and fills the job descriptors (scratch regions are carved out of
 // the context's scratch buffer, which is grown here when the stream is not capturing).
 int prepare_jobs(lmb_ctx *ctx, int kind, const LinearArgs *args, int njobs, Job *jobs, int *ctas_out, int *s_max_out,
@@ -1188,8 +1233,14 @@ int launch_gemv(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, in
       set_last_error("launch_gemv: jobs of one launch must share block kind and batch size");
       return LMB_ERR_ARG;
     }
-  if (batched_possible(args, njobs)) {
-    const int st = launch_batched(ctx, args, njobs, rotate, xmode, eps);
+  if (batched_possible(args, njobs) && (ctx->batched_force_seqs || batched_worth_asking(kind, args, njobs))) {
+    // From five sequences on the warp-level kernel takes 8 per pass and is behind at every measured shape (at best
+    // level: 2-bit 28672 x 2048, 5 sequences, 22.2 us against 21.3; other kinds 1.17 times and more).  With 3 or 4, which
+    // it takes in one pass of 4, and for the kinds that it serves two at a time without a conversion launch, the two
+    // estimates decide (1 % off the better kernel's time on average; both are wrong by 5 to 10 % at single shapes).
+    const bool compare = args[0].batch <= 4 || max_seqs_per_pass(kind) <= 2;
+    const int st = launch_batched(ctx, args, njobs, rotate, xmode, eps,
+                                  compare ? warp_level_us(kind, args, njobs, ctx->sm_count) : std::numeric_limits<float>::infinity());
     if (st != LMB_ERR_LIMIT) return st;
   }
   GemvParams p;
@@ -1249,11 +1300,18 @@ int launch_gemv(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, in
       }
     }
     if (need <= ctx->xprep_blocks) {
-      dim3 grid(unsigned((bpr + WARPS - 1) / WARPS), unsigned(args[0].batch));
-      k_prepare_x<<<grid, THREADS, 0, ctx->stream>>>(args[0].x, args[0].x2, unsigned(args[0].x_len), unsigned(args[0].x_stride),
-                                                     int(bpr), xmode, rotate ? 1 : 0, eps, ctx->xprep);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(unsigned((bpr + WARPS - 1) / WARPS), unsigned(args[0].batch));
+      cfg.blockDim = dim3(THREADS);
+      cfg.stream = ctx->stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = ctx->pdl ? 1 : 0;
+      LMB_CUDA(cudaLaunchKernelEx(&cfg, k_prepare_x, args[0].x, args[0].x2, unsigned(args[0].x_len), unsigned(args[0].x_stride), int(bpr), xmode,
+                                  rotate ? 1 : 0, eps, ctx->xprep));
       ctx->launches++;
-      LMB_CUDA(cudaGetLastError());
       p.prep = ctx->xprep;
     }
   }

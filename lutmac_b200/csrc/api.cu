@@ -427,7 +427,11 @@ int lmb_memset(lmb_ctx *ctx, void *d_dst, int value, size_t bytes) {
 
 int lmb_host_alloc_pinned(size_t bytes, void **h_ptr) {
   LMB_REQUIRE(h_ptr, "lmb_host_alloc_pinned: null argument");
-  LMB_CUDA(cudaMallocHost(h_ptr, bytes ? bytes : 1));
+  const cudaError_t e = cudaMallocHost(h_ptr, bytes ? bytes : 1);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // a caller that goes on with ordinary memory must not find this behind its next launch
+    return cuda_fail(e, "lmb_host_alloc_pinned");
+  }
   return LMB_OK;
 }
 

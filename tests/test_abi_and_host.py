@@ -186,3 +186,19 @@ def test_planner_cuts_launches_sensibly():
     # batches: 2, 4, 8 sequences per pass on the tensor-core kinds, 1 on the table-lookup kinds
     assert [_plan(INT2_MMA, 8960, 1536, b)["nseq"] for b in (1, 2, 3, 5, 32)] == [1, 2, 4, 8, 8]
     assert _plan(3, 8960, 1536, 8)["nseq"] == 1
+
+
+def test_logits_fall_back_to_ordinary_memory(monkeypatch):
+    """Where page-locking is refused the model's logits live in ordinary memory (the library's call fails as on a
+    machine with a limit on locked memory)."""
+    from lutmac_b200 import model
+
+    class Refuses:
+        @staticmethod
+        def lmb_host_alloc_pinned(n_bytes, out):
+            return _lib.ERR_CUDA
+
+    monkeypatch.setattr(model, "lib", lambda: Refuses)
+    a = model._pinned_floats(3, 50)
+    a[:] = 1.0
+    assert a.shape == (3, 50) and a.dtype == np.float32

@@ -62,6 +62,7 @@ struct BtParams {
   unsigned *fault;
   unsigned spin_limit;
   int extra_arrivals;   // test hook: the operand barriers expect this many arrivals too many
+  unsigned long long *dbg;  // this launch's slot of the launch timeline (debugging), or null
 #ifdef LMB_DEBUG_BOUNDS
   size_t scratch_floats;
 #endif
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
+    tl_min(p.dbg, 0);
     gave_up = 0;
     for (int s = 0; s < p.n_stages; ++s) {
       mbar_init(&full[s], 1);
@@ -310,6 +312,8 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
     // those kernels' run time (another rank's lateness among it) to this kernel's limit.
     pdl_wait();
     if (lane == 0) {
+      tl_min(p.dbg, 1);
+      tl_max(p.dbg, 2);
       const unsigned groups = unsigned(p.ns) / 2;  // 8-row groups of B: two sequences x four digits
       const uint32_t idesc = (2u << 4) | (KIND == DK_INT8_MMA ? 1u << 7 : 0u) | (1u << 10) | ((unsigned(p.ns) * 4u >> 3) << 17) | (8u << 24);
       const uint64_t lbo = groups * 128u >> 4, sbo = 128u >> 4;  // core matrices: [16-column chunk][8-row group][8 rows][16 bytes]
@@ -318,6 +322,7 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
       unsigned st_par = 0;
       for (int i = 0; i < n && ok; ++i) {
         ok = wait(&full[st], st_par);
+        if (i == 0) tl_max(p.dbg, 3);  // stamped here, not by the workers: they have no register to spare
         const uint64_t bdesc0 = (uint64_t(1) << 46) | (sbo << 32) | (lbo << 16) |
                                 uint64_t((smem_addr_u32(stages) + unsigned(st) * p.stage_bytes + B_OFF) >> 4);
         for (int pl = 0; pl < P && ok; ++pl) {
@@ -340,6 +345,7 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
       // no MMA is in flight when the TMEM is given back, whatever the workers have waited for
       tc_commit(&drain);
       for (unsigned s = 0; s < BT_DRAIN_POLLS && !mbar_try_wait(&drain, 0); ++s) {}
+      tl_max(p.dbg, 4);
     }
   } else {
     pdl_wait();
@@ -543,19 +549,31 @@ __global__ void __launch_bounds__(bt_threads(KIND), 512 / bt_tmem_cols(KIND, NSM
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == W + 1) tc_dealloc(tmem, COLS);
+  if (warp == W + 1) {
+    tc_dealloc(tmem, COLS);
+    if (lane == 0) {
+      tl_max(p.dbg, 5);
+      tl_min(p.dbg, 6);
+    }
+  }
 }
 
 // Operand images of a launch's activations: normalised / gated / rotated and cut into digits once.  One warp
 // per (sequence, block); grid = (ceil(bpr / 8), sequences).
 constexpr int BT_PREP_THREADS = 256;
 __global__ void __launch_bounds__(BT_PREP_THREADS) k_prepare_batched(const float *x, const float *x2, unsigned x_len, unsigned x_stride, int bpr,
-                                                                     int xmode, int rotate, float eps, int ns, uint8_t *img) {
+                                                                     int xmode, int rotate, float eps, int ns, uint8_t *img,
+                                                                     unsigned long long *dbg) {
   pdl_launch_dependents();
+  if (threadIdx.x == 0) tl_min(dbg, 0);
   __shared__ float red[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.y;
   const float *xq = x + size_t(q) * x_stride;
   pdl_wait();
+  if (threadIdx.x == 0) {
+    tl_min(dbg, 1);
+    tl_max(dbg, 2);
+  }
   float inv_rms = 1.0f;
   if (xmode == XMODE_RMSNORM) {  // src/layers/norm.cpp:18-34
     float ss = 0.0f;
@@ -585,6 +603,7 @@ __global__ void __launch_bounds__(BT_PREP_THREADS) k_prepare_batched(const float
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = (xmode == XMODE_GELU_MUL ? gelu_tanh(v[e]) : v[e] / (1.0f + expf(-v[e]))) * w8[e];
   }
+  if (threadIdx.x == 0) tl_max(dbg, 3);
   if (rotate) fwht256_warp(v, lane);
   MmaDigits dg;
   mma_digits(v, dg);
@@ -596,6 +615,11 @@ __global__ void __launch_bounds__(BT_PREP_THREADS) k_prepare_batched(const float
   for (int d = 0; d < 4; ++d) *reinterpret_cast<uint2 *>(dst + d * 16) = make_uint2(dg.words[d][0], dg.words[d][1]);
   if (lane == 0)
     *reinterpret_cast<int4 *>(im + size_t(ns) * 1024 + sq * 16) = make_int4(__float_as_int(dg.bscale), dg.d01, dg.d23, 0);
+  if (threadIdx.x == 0) {
+    tl_max(dbg, 4);
+    tl_max(dbg, 5);
+    tl_min(dbg, 6);
+  }
 }
 
 struct BtPlan {
@@ -805,8 +829,9 @@ int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate,
   cfg.attrs = attr;
   cfg.numAttrs = ctx->pdl ? 1 : 0;
   LMB_CUDA(cudaLaunchKernelEx(&cfg, k_prepare_batched, args[0].x, args[0].x2, unsigned(args[0].x_len), unsigned(args[0].x_stride), p.bpr, xmode,
-                              rotate ? 1 : 0, eps, p.ns, reinterpret_cast<uint8_t *>(ctx->xprep)));
+                              rotate ? 1 : 0, eps, p.ns, reinterpret_cast<uint8_t *>(ctx->xprep), timeline_slot(ctx)));
   ctx->launches++;
+  p.dbg = timeline_slot(ctx);
   switch (kind) {
   case LMB_INT4: return launch_kind<LMB_INT4>(ctx, p, pl);
   case DK_TERNARY_MMA: return launch_kind<DK_TERNARY_MMA>(ctx, p, pl);

@@ -146,7 +146,7 @@ template <int PER> __host__ __device__ constexpr size_t stream_smem_floats() {
 
 template <int PER, int G>
 __global__ void __launch_bounds__(STREAM_THREADS, 2) k_decode_attn_stream(const AttnArgs a, const RopeDims d, unsigned spin_limit, int extra_arrivals,
-                                                                          unsigned *timed_out) {
+                                                                          unsigned *timed_out, unsigned long long *tl) {
   constexpr int T = 32 / G, HD = 32 * PER, CH = stream_chunk<PER>(), ST = STREAM_STAGES;
   static_assert(CH % (STREAM_WARPS * T) == 0, "whole rounds");
   extern __shared__ __align__(128) float sm[];
@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_decode_attn_stream(const 
   const size_t kv_dim = d.nkv * HD;
   asm volatile("griddepcontrol.launch_dependents;");
   if (tid == 0) {
+    tl_min(tl, 0);
     gave_up = 0;
     for (int s = 0; s < ST; ++s) {
       mbar_init(&full[s], 1);
@@ -196,6 +197,10 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_decode_attn_stream(const 
   if (tid == 0)
     for (int c = 0; c < min(ST, n_chunks); ++c) fetch(c);  // written by earlier steps: not waited for
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (tid == 0) {
+    tl_min(tl, 1);
+    tl_max(tl, 2);
+  }
   // rotated queries of the group, and the new position (bias, RoPE; pairs (i, i + hd/2))
   constexpr int half = HD / 2;
   const float *cs = a.cs_table + pos * HD;
@@ -236,6 +241,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_decode_attn_stream(const 
     vc[pos * HD + j] = v0; vc[pos * HD + j + half] = v1;
   }
   __syncthreads();
+  if (tid == 0) tl_max(tl, 3);
   LaneVec<PER> q[G], acc[G];
 #pragma unroll
   for (int h = 0; h < G; ++h) {
@@ -392,6 +398,11 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_decode_attn_stream(const 
       }
     }
   }
+  if (tid == 0) {
+    tl_max(tl, 4);
+    tl_min(tl, 6);
+    tl_max(tl, 5);  // of the CTA that merges: again when it has
+  }
   if (n_splits == 1) return;
   __syncthreads();
   unsigned *ctr = a.counters + b * d.nkv + kvh;
@@ -439,6 +450,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_decode_attn_stream(const 
 #pragma unroll
   for (int e = 0; e < PER; ++e) tot.v[e] *= inv;
   st_lane_vec<PER>(a.out + (b * d.nh + head) * HD, lane, tot);
+  if (tid == 0) tl_max(tl, 5);
 }
 
 __global__ void k_interleave_rows(const float *src, float *dst, size_t ranks, size_t batch, size_t n) {
@@ -602,9 +614,9 @@ int launch_decode_attn_group(lmb_ctx *ctx, const float *q, const float *k, const
     cfg.gridDim = dim3(unsigned(d.nkv * size_t(a.n_splits)), unsigned(batch));
     cfg.dynamicSmemBytes = (plan.per == 4 ? stream_smem_floats<4>() : stream_smem_floats<2>()) * sizeof(float);
     // four query heads per KV head or fewer: eight positions per round instead of four
-    if (plan.per == 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<4, 8>, a, d, limit, extra, flag));
-    else if (d.nh / d.nkv > 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<2, 8>, a, d, limit, extra, flag));
-    else LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<2, 4>, a, d, limit, extra, flag));
+    if (plan.per == 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<4, 8>, a, d, limit, extra, flag, timeline_slot(ctx)));
+    else if (d.nh / d.nkv > 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<2, 8>, a, d, limit, extra, flag, timeline_slot(ctx)));
+    else LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_stream<2, 4>, a, d, limit, extra, flag, timeline_slot(ctx)));
   }
   ctx->launches++;
   return LMB_OK;

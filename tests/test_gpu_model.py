@@ -220,3 +220,32 @@ def test_launch_timeline_records_every_launch_of_a_step():
         if i:
             assert done >= int(t[i - 1][5]), (i, "finished before its predecessor")
     m.close()
+
+
+def test_launch_timeline_of_several_sequences():
+    """The same with 3 sequences, all projections on the batched kernel: two launches per projection call and one of
+    the streaming attention, 9 per layer, and 2 for the head; every launch has its slot."""
+    import ctypes as C
+    from lutmac_b200 import _lib
+    from lutmac_b200.api import Context
+    ctx = Context(0)
+    L = _lib.lib()
+    n = C.c_size_t()
+    _lib.check(L.lmb_debug_batched_plan(ctx.h, 8, 0))
+    _lib.check(L.lmb_debug_launch_timeline(ctx.h, 256, None, C.byref(n)))
+    m = Model(synth.model_spec(synth.tiny_model_shape(n_layers=3), INT4, seed=2, max_seq=16), ctx, max_batch=3)
+    for p in range(3):
+        m.forward([7, 8, 9], [p] * 3)
+    _lib.check(L.lmb_debug_launch_timeline(ctx.h, 0, None, C.byref(n)))  # clears what the steps so far recorded
+    m.forward([1, 2, 3], [3] * 3)
+    out = (C.c_uint64 * (8 * 256))()
+    _lib.check(L.lmb_debug_launch_timeline(ctx.h, 0, out, C.byref(n)))
+    assert n.value == 9 * 3 + 2
+    t = np.array(list(out)[:8 * n.value], np.uint64).reshape(n.value, 8)
+    for i in range(n.value):
+        start, first_wait, last_wait, ready, main, done, first_done = (int(t[i][k]) for k in range(7))
+        assert 0 < start <= first_wait <= last_wait <= ready <= main <= done, (i, t[i])
+        assert first_wait <= first_done <= done + 1000, (i, t[i])
+        if i:
+            assert done >= int(t[i - 1][5]), (i, "finished before its predecessor")
+    m.close()

@@ -434,7 +434,7 @@ template <int PER> __device__ __forceinline__ LaneVec<PER> ldcg_lane_vec(const f
 // for the copies (dbg[0]) and after the partial records are written (dbg[1]).
 // WIDE: the form for batch 1, where the kernel is one wave of CTAs and bound by their latency: queries
 // kept in registers, the value pass by timestep with all heads per lane, merge statistics in one round
-// trip and 16 partial records in flight.  With several sequences (many waves) the plain form is faster.
+// trip and 16 partial records in flight.  The plain form (fewer registers) serves the persistent step.
 template <bool FRESH_CG, int PER, bool WIDE = false>
 __device__ __forceinline__ bool attn_group_item(const AttnArgs &a, const RopeDims &d, size_t kvh, size_t split, size_t b, float *sm,
                                                 uint64_t *bar, unsigned &parity, unsigned spin_limit, int *flag,

@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn(const AttnArgs a, c
   attn_item<false>(a, d, blockIdx.x, blockIdx.y, blockIdx.z, sm, &is_last);
 }
 
-// Group attention as a kernel of its own: grid = (KV heads x splits, sequences).
-template <int PER, bool WIDE>
+// Group attention of one sequence as a kernel of its own: grid = (KV heads x splits, 1).
+template <int PER>
 __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn_group(const AttnArgs a, const RopeDims d, unsigned spin_limit,
                                                                     unsigned *timed_out, unsigned long long *tl) {
   asm volatile("griddepcontrol.launch_dependents;");
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn_group(const AttnArg
   __syncthreads();
   unsigned parity = 0;
   const size_t kvh = blockIdx.x % d.nkv, split = blockIdx.x / d.nkv;
-  if (!attn_group_item<false, PER, WIDE>(a, d, kvh, split, blockIdx.y, sm, &bar, parity, spin_limit, &flag, nullptr, tl) && threadIdx.x == 0 &&
+  if (!attn_group_item<false, PER, true>(a, d, kvh, split, blockIdx.y, sm, &bar, parity, spin_limit, &flag, nullptr, tl) && threadIdx.x == 0 &&
       timed_out)
     *timed_out = 1u;
 }
@@ -602,11 +602,12 @@ int launch_decode_attn_group(lmb_ctx *ctx, const float *q, const float *k, const
     return !(e && e[0] == '0');
   }();
   cfg.numAttrs = ctx->pdl && attn_pdl ? 1 : 0;
-  // one sequence: one wave of CTAs, bound by their latency (the WIDE form); several: bound by throughput (the streaming form)
+  // one sequence: one wave of CTAs, bound by their latency; several: bound by throughput (the streaming form, which
+  // takes nothing of `plan` but the head size: it has splits of its own, of any length)
   if (batch == 1) {
     unsigned long long *tl = timeline_slot(ctx);
-    if (plan.per == 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_group<4, true>, a, d, ctx->xchg.spin_limit, flag, tl));
-    else LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_group<2, true>, a, d, ctx->xchg.spin_limit, flag, tl));
+    if (plan.per == 4) LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_group<4>, a, d, ctx->xchg.spin_limit, flag, tl));
+    else LMB_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_group<2>, a, d, ctx->xchg.spin_limit, flag, tl));
   } else {
     a.n_splits = ctx->attn_force_splits ? ctx->attn_force_splits : stream_splits(d.nkv, batch, d.max_seq, size_t(ctx->sm_count));
     const unsigned limit = ctx->attn_spin_limit ? ctx->attn_spin_limit : ctx->xchg.spin_limit;
@@ -639,8 +640,8 @@ int launch_silu_mul(lmb_ctx *ctx, const float *gate, const float *up, float *out
 
 int configure_decode_ops(lmb_ctx *ctx) {
   LMB_CUDA(cudaFuncSetAttribute(k_decode_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ctx->smem_optin) - 1024));
-  LMB_CUDA(cudaFuncSetAttribute(k_decode_attn_group<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ATTN_GROUP_SMEM)));
-  LMB_CUDA(cudaFuncSetAttribute(k_decode_attn_group<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ATTN_GROUP_SMEM)));
+  LMB_CUDA(cudaFuncSetAttribute(k_decode_attn_group<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ATTN_GROUP_SMEM)));
+  LMB_CUDA(cudaFuncSetAttribute(k_decode_attn_group<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ATTN_GROUP_SMEM)));
   LMB_CUDA(cudaFuncSetAttribute(k_decode_attn_stream<4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(stream_smem_floats<4>() * 4)));
   LMB_CUDA(cudaFuncSetAttribute(k_decode_attn_stream<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(stream_smem_floats<2>() * 4)));
   LMB_CUDA(cudaFuncSetAttribute(k_decode_attn_stream<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(stream_smem_floats<2>() * 4)));

@@ -175,3 +175,61 @@ def test_step_after_an_expired_attention_wait(ctx, oracle, head_dim, pos, monkey
     finally:
         _lib.check(L.lmb_debug_attn_stream(ctx.h, 0, 0, 0))
     m.close()
+
+
+@pytest.mark.parametrize("splits", (1, 3))
+@pytest.mark.parametrize("head_dim,n_heads,n_kv", [(64, 8, 2), (64, 6, 1), (128, 4, 2)])
+def test_batched_attention_refills_its_ring(ctx, oracle, head_dim, n_heads, n_kv, splits, monkeypatch):
+    """Four to six chunks per split through the ring of three stages, in each of the three forms: refills, phase
+    flips and a ragged tail behind full chunks, over a random cache."""
+    monkeypatch.setenv("LMB_MODEL_GRAPH", "0")
+    L = _lib.lib()
+    chunk = splits * (32 if head_dim == 128 else 64)
+    start = [5 * chunk - 1, 4 * chunk - 2, 3 * chunk + 7]
+    spec, m, refs, rng = _models_with_context(ctx, oracle, head_dim, n_heads, n_kv, start, 23)
+    try:
+        _lib.check(L.lmb_debug_attn_stream(ctx.h, splits, 0, 0))
+        for s in range(4):
+            toks, pos = rng.integers(0, spec.cfg["vocab"], size=3).astype(np.int32), [p + s for p in start]
+            got = m.forward(toks, pos)
+            for q in range(3):
+                assert rel_l2(got[q], refs[q].forward(int(toks[q]), pos[q])) < 1e-5, (s, q)
+    finally:
+        _lib.check(L.lmb_debug_attn_stream(ctx.h, 0, 0, 0))
+    m.close()
+
+
+# (sequences, sequences per pass, CTAs per pass): every accumulator form with all units of the launch in one CTA (20 to
+# 60 units, ranges over several row groups, every stage reused, sums folded every 8 blocks), ranges that end inside a
+# row group, several passes, and as many CTAs as there are units
+PLANS = [(3, 4, 1), (8, 8, 3), (16, 16, 1), (17, 32, 2), (32, 32, 1), (32, 8, 2), (9, 16, 1000), (31, 32, 7)]
+
+
+@pytest.mark.parametrize("kind", (TERNARY, BINARY, INT2, INT3, INT4, INT5, INT6, INT8))
+def test_batched_long_ranges_vs_fp64(ctx, oracle, kind):
+    """Odd strides (rows that are not 16-byte aligned), a bias, and every plan of PLANS."""
+    L = _lib.lib()
+    rng = np.random.default_rng(70 + kind)
+    M, K = 300, 5000
+    t = synth.tensor(rng, kind, M, K)
+    w, stride = ctx.upload(t), K + 3
+    bias = rng.standard_normal(M).astype(np.float32)
+    db = ctx.to_device(bias)
+    for batch, seqs, ctas in PLANS:
+        x = np.stack([synth.activations(rng, stride) for _ in range(batch)])
+        dx, dy = ctx.to_device(x), ctx.malloc(batch * M * 4)
+        _lib.check(L.lmb_debug_batched_plan(ctx.h, seqs, ctas))
+        try:
+            for _ in range(2):  # twice: the arrival counters must be back at zero
+                dy.zero()
+                ctx.linear(w, dx, dy, batch=batch, bias=db, flags=0, x_len=K, x_stride=stride)
+                y = dy.download(np.float32).reshape(batch, M)
+        finally:
+            _lib.check(L.lmb_debug_batched_plan(ctx.h, 0, 0))
+        for q in sorted({0, 1, batch // 2, batch - 1}):
+            padded = np.zeros(blocks_per_row(K) * 256, np.float32)
+            padded[:K] = x[q, :K]
+            want = oracle.gemv_f64(kind, t.blocks, padded, M, K) + bias
+            err = np.linalg.norm(y[q] - want)
+            assert err < TOL * np.linalg.norm(np.abs(want) + 1e-3 * np.linalg.norm(padded)), (batch, seqs, ctas, q, err)
+    w.free()

@@ -97,7 +97,10 @@ int lmb_timer_stop(lmb_ctx *ctx, float *ms_out); /* records, synchronises, retur
 
 /* CUDA-graph capture of the work a context issues (kernel launches only; no host-pointer entry
  * point may be called while capturing).  lmb_graph_end returns an executable graph that
- * lmb_graph_launch replays on the context's stream. */
+ * lmb_graph_launch replays on the context's stream.  Issue the calls once before capturing them: workspaces cannot
+ * grow during a capture, so a launch that needs more split-K scratch fails there, and one of several sequences whose
+ * operand images do not fit takes the warp-level kernel, which the graph then keeps (the same result up to the order
+ * of fp32 sums, more slowly). */
 typedef struct lmb_graph lmb_graph;
 int lmb_graph_begin(lmb_ctx *ctx);
 int lmb_graph_end(lmb_ctx *ctx, lmb_graph **out);
@@ -226,7 +229,8 @@ int lmb_debug_plan_weight(const lmb_weight *w, int sm_count, int out5[5]);
  * Process-wide; graphs captured earlier keep their plans. */
 int lmb_debug_force_plan(int R, int n_ks, int cr);
 /* Tests: from now on the batched projections' operand barriers expect `extra_arrivals` arrivals too many
- * and their waits give up after `spin_limit` polls (0: the default); 0, 0: off. */
+ * and their waits give up after `spin_limit` polls (0: the default); 0, 0: off.  With extra arrivals every launch that
+ * the batched kernel can serve takes it, as with lmb_debug_batched_plan. */
 int lmb_debug_batched_waits(lmb_ctx *ctx, int extra_arrivals, unsigned spin_limit);
 /* Tests: from now on the batched projections take this many sequences per pass (a multiple of 4 up to 32) and
  * this many CTAs per pass (no more than there are units of work); 0: the planner's choice. */

@@ -13,7 +13,7 @@
 //
 // What bounds it: warp-level IMMA re-read the weights once per 8 sequences and spent 16 MMAs, their
 // operand loads and the scaling of every (32 rows x 2 sequences) in the same warps; here the weights are
-// read once per 32 sequences and the tensor work leaves the warps, which keep the byte expansion
+// read once per 8, 16 or 32 sequences and the tensor work leaves the warps, which keep the byte expansion
 // (64 masks per 32 x 256 codes) and the scaling (9 instructions per row, sequence and block).  Ternary
 // 8192 x 28672, 16 sequences: 133 us before, 44 us with this kernel (9.9 us of HBM time).  Measured on the way
 // and not taken: two warps per tile (46 us; 24 instead of 19 us at 8192 x 8192).  With an eighth of the MMAs,
@@ -21,8 +21,8 @@
 // of the bytes 42 us: what is left is the chain of expansion, hand-over and scaling inside a warp.
 //
 // Work split: the (row group, block) units of all jobs of a launch are one flat list, cut into equal
-// contiguous ranges, one per CTA, whatever the shapes: no nearly empty last wave.  A row group whose
-// blocks lie in several CTAs is added up, in CTA order, by the warp that arrives last.
+// contiguous ranges, one per CTA; how many CTAs, and how many passes over the sequences, plan_batched
+// decides.  A row group whose blocks lie in several CTAs is added up, in CTA order, by the warp that arrives last.
 //
 // Roles: 4 * H worker warps (a 32-row tile each), one producer thread (bulk copies), one MMA thread.
 // Every wait is bounded: on expiry the kernel raises the context's fault flag and leaves in order.
@@ -774,7 +774,7 @@ int launch_batched(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate,
   size_t row_tiles[BT_MAX_JOBS];
   for (int j = 0; j < njobs; ++j) row_tiles[j] = args[j].w->row_tiles;
   const BtPlan pl = plan_batched(kind, row_tiles, njobs, args[0].w->bpr, args[0].batch, ctx->sm_count, ctx->batched_force_seqs, ctx->batched_force_ctas);
-  if (pl.n_stages < 2 || (pl.us > limit_us && !ctx->batched_force_seqs)) return LMB_ERR_LIMIT;
+  if (pl.n_stages < 2 || pl.us > limit_us) return LMB_ERR_LIMIT;
   if (pl.scratch > ctx->scratch_floats || pl.counters > ctx->n_counters || pl.img_records > ctx->xprep_blocks) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     LMB_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));

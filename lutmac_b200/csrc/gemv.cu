@@ -22,7 +22,8 @@
 // 256-column blocks).  A warp streams weight tiles with 128-bit coalesced loads through a ring
 // of register slots.  When K is split over several CTAs, partial sums go to a scratch buffer
 // and the last CTA to arrive for a row group adds them in slice order (deterministic).
-// Batches: 2, 4 or 8 sequences share one pass over the weights on the tensor-core units.
+// Batches: 2, 4 or 8 sequences share one pass over the weights on the tensor-core units; most launches of three or
+// more go to the kernel in batched.cu (see launch_gemv).
 //
 // Programmatic dependent launch: a kernel lets its successor start at once, the successor
 // prefetches its first weight tiles (weights never depend on a predecessor) and only then
@@ -193,8 +194,8 @@ __global__ void __launch_bounds__(THREADS, min_ctas(KIND, NSEQ)) k_gemv(const __
   float *inv_rms = part[0];  // [sequence] after the block below (XMODE_RMSNORM)
   // One sequence: RMSNorm (src/layers/norm.cpp:18-34) is linear in 1 / rms, so the digits below are those of
   // x * w and the row sums are multiplied by 1 / rms at the end: the sum of squares and the conversion read x
-  // side by side, instead of one round trip and two barriers after the other (1B-shaped step with the
-  // page-locked logits: 611 -> 558 us).
+  // side by side, instead of one round trip and two barriers after the other (4 layers of a 1B shape and the head,
+  // us a step: ternary 152 -> 145, 2-bit 153 -> 148, 4-bit 142 -> 140).
   const bool late_rms = !ALONE && NSEQ == 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered;
   if (NSEQ > 1 && p.xmode == XMODE_RMSNORM && !p.prep && !clustered) {
     // RMSNorm of the whole input vectors, recomputed by every CTA
@@ -1233,12 +1234,13 @@ int launch_gemv(lmb_ctx *ctx, const LinearArgs *args, int njobs, bool rotate, in
       set_last_error("launch_gemv: jobs of one launch must share block kind and batch size");
       return LMB_ERR_ARG;
     }
-  if (batched_possible(args, njobs) && (ctx->batched_force_seqs || batched_worth_asking(kind, args, njobs))) {
+  const bool forced = ctx->batched_force_seqs || ctx->batched_extra_arrivals;  // test hooks
+  if (batched_possible(args, njobs) && (forced || batched_worth_asking(kind, args, njobs))) {
     // From five sequences on the warp-level kernel takes 8 per pass and is behind at every measured shape (at best
     // level: 2-bit 28672 x 2048, 5 sequences, 22.2 us against 21.3; other kinds 1.17 times and more).  With 3 or 4, which
     // it takes in one pass of 4, and for the kinds that it serves two at a time without a conversion launch, the two
     // estimates decide (1 % off the better kernel's time on average; both are wrong by 5 to 10 % at single shapes).
-    const bool compare = args[0].batch <= 4 || max_seqs_per_pass(kind) <= 2;
+    const bool compare = !forced && (args[0].batch <= 4 || max_seqs_per_pass(kind) <= 2);
     const int st = launch_batched(ctx, args, njobs, rotate, xmode, eps,
                                   compare ? warp_level_us(kind, args, njobs, ctx->sm_count) : std::numeric_limits<float>::infinity());
     if (st != LMB_ERR_LIMIT) return st;

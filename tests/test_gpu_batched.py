@@ -104,10 +104,11 @@ def test_batched_limit_does_not_count_the_kernels_before(ctx):
     t = synth.int4_tensor(rng, 256, 256)
     x = np.stack([synth.activations(rng, 256) for _ in range(4)])
     w, dx, dy, dy2 = ctx.upload(t), ctx.to_device(x), ctx.malloc(4 * 256 * 4), ctx.malloc(4 * 256 * 4)
-    ctx.linear(w, dx, dy2, batch=4)
-    want = dy2.download(np.float32)
-    dy2.zero()
     try:
+        _lib.check(L.lmb_debug_batched_plan(ctx.h, 4, 1))
+        ctx.linear(w, dx, dy2, batch=4)
+        want = dy2.download(np.float32)
+        dy2.zero()
         _lib.check(L.lmb_debug_batched_waits(ctx.h, 1, 100000))
         ctx.linear(w, dx, dy, batch=4)
         _lib.check(L.lmb_debug_batched_waits(ctx.h, 0, 2000))
@@ -117,6 +118,7 @@ def test_batched_limit_does_not_count_the_kernels_before(ctx):
         assert e.value.status == _lib.ERR_TIMEOUT
     finally:
         _lib.check(L.lmb_debug_batched_waits(ctx.h, 0, 0))
+        _lib.check(L.lmb_debug_batched_plan(ctx.h, 0, 0))
     assert np.array_equal(dy2.download(np.float32), want)
     w.free()
 

